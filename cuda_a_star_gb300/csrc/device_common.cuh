@@ -63,6 +63,13 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// A value that is the same in every lane, as a warp reduction's result.  The
+// compiler takes what a load, a shuffle or threadIdx yields for per-lane data
+// and guards every branch on it with convergence code; the result of a
+// reduction or a vote is uniform to it, and so are the branches.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __reduce_or_sync(kFull, v); }
+__device__ __forceinline__ bool uniform_if(bool c) { return __any_sync(kFull, c) != 0; }
+
 // ---------------------------------------------------------------------------
 // Heap entries: a priority word and KW 64-bit key words (KW = 1..4), padded to
 // a multiple of 16 bytes: 16 B for 64-bit keys, 32 B for 128..192-bit keys,
@@ -132,8 +139,8 @@ template <int KW> __device__ __forceinline__ void st_entry(Entry<KW>* p, const E
 // Stage-buffer access: shared memory for one-block teams (plain generic
 // accesses), global memory shared by the blocks of a multi-block team
 // (L2-coherent accesses, since the buffer is refilled every iteration).
-template <int KW> __device__ __forceinline__ Entry<KW> ld_stage(const Entry<KW>* p, bool global) {
-    if (global) return ld_entry(p);
+template <bool GLOBAL, int KW> __device__ __forceinline__ Entry<KW> ld_stage(const Entry<KW>* p) {
+    if constexpr (GLOBAL) return ld_entry(p);
     Entry<KW> e;
     const uint4* s = reinterpret_cast<const uint4*>(p);
 #pragma unroll
@@ -144,8 +151,8 @@ template <int KW> __device__ __forceinline__ Entry<KW> ld_stage(const Entry<KW>*
     }
     return e;
 }
-template <int KW> __device__ __forceinline__ void st_stage(Entry<KW>* p, const Entry<KW>& e, bool global) {
-    if (global) {
+template <bool GLOBAL, int KW> __device__ __forceinline__ void st_stage(Entry<KW>* p, const Entry<KW>& e) {
+    if constexpr (GLOBAL) {
         st_entry(p, e);
         return;
     }
@@ -214,11 +221,15 @@ __device__ __forceinline__ Entry<KW> pick(const Entry<KW>& lo, const Entry<KW>& 
 //
 // One warp owns one heap.  A node holds 32 entries sorted ascending; the heap
 // order is node-wise (every entry of a node <= every entry of its children),
-// so the root holds the 32 best entries of the tree.  The root node and a
-// partial buffer of < 32 entries live in registers (one entry per lane) for
-// the lifetime of a launch, nodes 1..sn-1 in shared memory (the top levels;
-// sn is chosen per launch from the shared memory left on the SM), the rest are 512-byte (or 1 KiB) blocks in global memory read and written with
-// one coalesced access per lane.  Replaces the reference's one-thread-per-heap
+// so the root holds the 32 best entries of the tree.  A partial buffer of
+// < 32 entries and nodes 0..sn-1 (the top levels; sn is chosen per launch
+// from the shared memory left on the SM) live in shared memory for the
+// lifetime of a launch, the rest are 512-byte (or 1 KiB) blocks in global
+// memory read and written with one coalesced access per lane.  Root and
+// buffer stay out of registers: they are touched a few times per iteration,
+// and the 16-warp kernel has 128 registers per thread (holding them there
+// spilled ~500 bytes per thread, whose local-memory traffic was 15x the
+// search's own loads).  Replaces the reference's one-thread-per-heap
 // binary heaps with their key->slot index (heaps.h:93-177, device_hashmap.h):
 // stale entries are dropped at pop time instead of being erased (lazy
 // deletion).
@@ -226,30 +237,33 @@ __device__ __forceinline__ Entry<KW> pick(const Entry<KW>& lo, const Entry<KW>& 
 
 template <int KW> struct WarpHeap {
     Entry<KW>* nodes;   // (cap + 1) * 32 entries; node `cap` stores the saved partial buffer
-    Entry<KW>* snodes;  // shared memory: nodes 1..sn-1
-    uint32_t* hdr;      // saved {N, pc}
+    Entry<KW>* snodes;  // shared memory: the partial buffer, then nodes 0..sn-1
     uint32_t cap;       // tree nodes available (>= sn)
-    uint32_t sn;        // nodes below sn live in shared memory (node 0 in registers)
+    uint32_t sn;        // nodes below sn live in shared memory
     uint32_t N;         // full nodes in the tree (warp-uniform)
-    uint32_t pc;        // entries in the partial buffer (warp-uniform)
+    uint32_t pc;        // entries in the partial buffer (warp-uniform), ascending; inf entries after
     uint32_t max_n;     // high-water mark of N
-    Entry<KW> root;     // lane l: root[l] (valid iff N > 0)
-    Entry<KW> part;     // lane l: partial[l] (valid iff l < pc), ascending
 };
 
+template <int KW> __device__ __forceinline__ Entry<KW> ld_part(const WarpHeap<KW>& h, int lane) {
+    return ld_stage<false>(h.snodes + lane);
+}
+template <int KW> __device__ __forceinline__ void st_part(const WarpHeap<KW>& h, int lane, const Entry<KW>& e) {
+    st_stage<false>(h.snodes + lane, e);
+}
 template <int KW>
 __device__ __forceinline__ Entry<KW> ld_node(const WarpHeap<KW>& h, uint32_t idx, int lane) {
-    if (idx < h.sn) return ld_stage(h.snodes + (size_t)(idx - 1) * 32 + lane, false);
+    if (idx < h.sn) return ld_stage<false>(h.snodes + (idx + 1) * 32 + lane);
     return ld_entry(h.nodes + (size_t)idx * 32 + lane);
 }
 template <int KW>
 __device__ __forceinline__ void st_node(const WarpHeap<KW>& h, uint32_t idx, int lane, const Entry<KW>& e) {
-    if (idx < h.sn) st_stage(h.snodes + (size_t)(idx - 1) * 32 + lane, e, false);
+    if (idx < h.sn) st_stage<false>(h.snodes + (idx + 1) * 32 + lane, e);
     else st_entry(h.nodes + (size_t)idx * 32 + lane, e);
 }
 // Priority of the largest entry of node idx (one read, broadcast to the warp).
 template <int KW> __device__ __forceinline__ uint64_t node_max(const WarpHeap<KW>& h, uint32_t idx) {
-    if (idx < h.sn) return *reinterpret_cast<const volatile uint64_t*>(&h.snodes[(size_t)(idx - 1) * 32 + 31].prio);
+    if (idx < h.sn) return *reinterpret_cast<const volatile uint64_t*>(&h.snodes[(idx + 1) * 32 + 31].prio);
     return __ldcg(reinterpret_cast<const unsigned long long*>(&h.nodes[(size_t)idx * 32 + 31].prio));
 }
 
@@ -262,48 +276,44 @@ template <int KW> __device__ __forceinline__ void prefetch_node(const WarpHeap<K
     }
 }
 
-template <int KW> __device__ __forceinline__ void heap_init(WarpHeap<KW>& h) {
+template <int KW> __device__ __forceinline__ void heap_init(WarpHeap<KW>& h, int lane) {
     h.N = 0;
     h.pc = 0;
     h.max_n = 0;
-    h.root = inf_entry<KW>();
-    h.part = inf_entry<KW>();
+    st_part(h, lane, inf_entry<KW>());
+    __syncwarp();
 }
 
-template <int KW> __device__ __forceinline__ void heap_restore(WarpHeap<KW>& h, int lane) {
-    h.N = __ldcg(h.hdr);
-    h.pc = __ldcg(h.hdr + 1);
+// `hdr`: the heap's saved {N, pc}.
+template <int KW> __device__ __forceinline__ void heap_restore(WarpHeap<KW>& h, const uint32_t* hdr, int lane) {
+    h.N = uniform(__ldcg(hdr));
+    h.pc = uniform(__ldcg(hdr + 1));
     h.max_n = h.N;
-    h.root = h.N ? ld_entry(h.nodes + lane) : inf_entry<KW>();
-    h.part = (uint32_t)lane < h.pc ? ld_entry(h.nodes + (size_t)h.cap * 32 + lane) : inf_entry<KW>();
-    for (uint32_t i = 1; i < h.N && i < h.sn; ++i)
-        st_stage(h.snodes + (size_t)(i - 1) * 32 + lane, ld_entry(h.nodes + (size_t)i * 32 + lane), false);
+    st_part(h, lane, (uint32_t)lane < h.pc ? ld_entry(h.nodes + (size_t)h.cap * 32 + lane) : inf_entry<KW>());
+    for (uint32_t i = 0; i < h.N && i < h.sn; ++i) st_node(h, i, lane, ld_entry(h.nodes + (size_t)i * 32 + lane));
     __syncwarp();
 }
 
-template <int KW> __device__ __forceinline__ void heap_save(const WarpHeap<KW>& h, int lane) {
+template <int KW> __device__ __forceinline__ void heap_save(const WarpHeap<KW>& h, uint32_t* hdr, int lane) {
     __syncwarp();
-    if (h.N) st_entry(h.nodes + lane, h.root);
-    for (uint32_t i = 1; i < h.N && i < h.sn; ++i)
-        st_entry(h.nodes + (size_t)i * 32 + lane, ld_stage(h.snodes + (size_t)(i - 1) * 32 + lane, false));
-    st_entry(h.nodes + (size_t)h.cap * 32 + lane, h.part);
+    for (uint32_t i = 0; i < h.N && i < h.sn; ++i) st_entry(h.nodes + (size_t)i * 32 + lane, ld_node(h, i, lane));
+    st_entry(h.nodes + (size_t)h.cap * 32 + lane, ld_part(h, lane));
     if (lane == 0) {
-        __stcg(h.hdr, h.N);
-        __stcg(h.hdr + 1, h.pc);
+        __stcg(hdr, h.N);
+        __stcg(hdr + 1, h.pc);
     }
 }
 
+// Least priority of the heap (kInfPrio when it is empty; the warp calls it
+// after the last change is visible to every lane).
 template <int KW> __device__ __forceinline__ uint64_t heap_min(const WarpHeap<KW>& h) {
-    uint64_t r = __shfl_sync(kFull, h.root.prio, 0);
-    uint64_t p = __shfl_sync(kFull, h.part.prio, 0);
-    r = h.N ? r : kInfPrio;
-    p = h.pc ? p : kInfPrio;
+    const uint64_t r = h.N ? *reinterpret_cast<const volatile uint64_t*>(&h.snodes[32].prio) : kInfPrio;
+    const uint64_t p = h.pc ? *reinterpret_cast<const volatile uint64_t*>(&h.snodes[0].prio) : kInfPrio;
     return r < p ? r : p;
 }
 
-// Restores the node order below the root after the root's content changed.
-template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, int lane) {
-    Entry<KW> cur = h.root;
+// Restores the node order from the root (new content `cur`, not stored yet) down.
+template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, Entry<KW> cur, int lane) {
     uint32_t idx = 0;
     for (;;) {
         uint32_t l = 2 * idx + 1, r = l + 1;
@@ -317,7 +327,7 @@ template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, int lane) {
         uint64_t cmax = __shfl_sync(kFull, cur.prio, 31);
         uint64_t lmin = __shfl_sync(kFull, L.prio, 0);
         if (r >= h.N) {
-            if (cmax > lmin) {
+            if (uniform_if(cmax > lmin)) {
                 Entry<KW> lo, hi;
                 merge2(cur, L, lo, hi, lane);
                 st_node(h, l, lane, hi);
@@ -327,22 +337,21 @@ template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, int lane) {
         }
         Entry<KW> R = ld_node(h, r, lane);
         uint64_t rmin = __shfl_sync(kFull, R.prio, 0);
-        if (cmax <= (lmin < rmin ? lmin : rmin)) break;
+        if (uniform_if(cmax <= (lmin < rmin ? lmin : rmin))) break;
         uint64_t lmax = __shfl_sync(kFull, L.prio, 31);
         uint64_t rmax = __shfl_sync(kFull, R.prio, 31);
         Entry<KW> A, B;
         merge2(L, R, A, B, lane);
-        uint32_t big = lmax >= rmax ? l : r, small = big == l ? r : l;
+        const bool left = uniform_if(lmax >= rmax);
+        const uint32_t big = left ? l : r, small = left ? r : l;
         st_node(h, big, lane, B);  // B.max = max(lmax, rmax): big's subtree stays ordered
         Entry<KW> lo, hi;
         merge2(cur, A, lo, hi, lane);
-        if (idx == 0) h.root = lo;
-        else st_node(h, idx, lane, lo);
+        st_node(h, idx, lane, lo);
         cur = hi;
         idx = small;
     }
-    if (idx == 0) h.root = cur;
-    else st_node(h, idx, lane, cur);
+    st_node(h, idx, lane, cur);
     __syncwarp();
 }
 
@@ -350,18 +359,20 @@ template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, int lane) {
 // l < return value receives one.  Nothing changes when no entry qualifies.
 template <int KW>
 __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW>& out, int lane) {
+    const Entry<KW> part = ld_part(h, lane);
     if (h.N == 0) {
-        const uint32_t below = __popc(__ballot_sync(kFull, (uint32_t)lane < h.pc && h.part.prio < lim));
+        const uint32_t below = __popc(__ballot_sync(kFull, (uint32_t)lane < h.pc && part.prio < lim));
         const uint32_t c = E < below ? E : below;
-        out = (uint32_t)lane < c ? h.part : inf_entry<KW>();
-        Entry<KW> s = shfl_idx(h.part, (lane + (int)c) & 31);
-        h.part = ((uint32_t)lane + c < h.pc) ? s : inf_entry<KW>();
+        out = (uint32_t)lane < c ? part : inf_entry<KW>();
+        Entry<KW> s = shfl_idx(part, (lane + (int)c) & 31);
+        st_part(h, lane, ((uint32_t)lane + c < h.pc) ? s : inf_entry<KW>());
         h.pc -= c;
+        __syncwarp();
         return c;
     }
     prefetch_node(h, h.N - 1, lane);  // the last node refills the root when the buffer runs short
     Entry<KW> lo, hi;
-    merge2(h.root, h.part, lo, hi, lane);
+    merge2(ld_node(h, 0, lane), part, lo, hi, lane);
     {
         const uint32_t below = __popc(__ballot_sync(kFull, lo.prio < lim));
         if (below < E) E = below;
@@ -378,24 +389,22 @@ __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW
     if ((uint32_t)i1 >= valid) r1 = inf_entry<KW>();
     if ((uint32_t)i2 >= valid) r2 = inf_entry<KW>();
     if (rest >= 32) {
-        h.root = r1;
-        h.part = r2;
+        st_part(h, lane, r2);
         h.pc = rest - 32;
-        heap_sift_down(h, lane);
+        heap_sift_down(h, r1, lane);
     } else if (h.N == 1) {
         h.N = 0;
-        h.root = inf_entry<KW>();
-        h.part = r1;
+        st_part(h, lane, r1);
         h.pc = rest;
+        __syncwarp();
     } else {
         Entry<KW> last = ld_node(h, h.N - 1, lane);
         h.N -= 1;
         Entry<KW> lo2, hi2;
         merge2(last, r1, lo2, hi2, lane);
-        h.root = lo2;
-        h.part = hi2;
+        st_part(h, lane, hi2);
         h.pc = rest;
-        heap_sift_down(h, lane);
+        heap_sift_down(h, lo2, lane);
     }
     return E;
 }
@@ -403,40 +412,26 @@ __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW
 // Adds a full node top-down along the path to the new leaf: every node on the
 // path keeps the 32 smallest of itself and the carried node.
 template <int KW> __device__ bool heap_insert_node(WarpHeap<KW>& h, Entry<KW> F, int lane) {
-    if (h.N == 0) {
-        h.root = F;
-        h.N = 1;
-        if (h.max_n < 1) h.max_n = 1;
-        return true;
-    }
     if (h.N >= h.cap) return false;
-    const uint32_t p = h.N + 1;
-    const int levels = 31 - __clz(p);
-    {
-        uint64_t fmin = __shfl_sync(kFull, F.prio, 0);
-        uint64_t rmax = __shfl_sync(kFull, h.root.prio, 31);
-        if (fmin < rmax) {
-            Entry<KW> lo, hi;
-            merge2(h.root, F, lo, hi, lane);
-            h.root = lo;
-            F = hi;
-        }
-    }
-    // The path is fixed by the new leaf's index: fetch the maximum of every
-    // node on it in one parallel load (lane j <- depth j), so only the nodes
-    // that need a merge cost a dependent access.
-    uint64_t pmax = kInfPrio;
-    if (lane >= 1 && lane < levels) pmax = node_max(h, (p >> (levels - lane)) - 1);
-    for (int b = levels - 1; b >= 1; --b) prefetch_node(h, (p >> b) - 1, lane);  // the nodes themselves
-    for (int b = levels - 1; b >= 1; --b) {
-        const uint32_t idx = (p >> b) - 1;
-        uint64_t fmin = __shfl_sync(kFull, F.prio, 0);
-        if (fmin < __shfl_sync(kFull, pmax, levels - b)) {
-            Entry<KW> M = ld_node(h, idx, lane);
-            Entry<KW> lo, hi;
-            merge2(M, F, lo, hi, lane);
-            st_node(h, idx, lane, lo);
-            F = hi;
+    if (h.N) {
+        const uint32_t p = h.N + 1;
+        const int levels = 31 - __clz(p);
+        // The path is fixed by the new leaf's index: fetch the maximum of
+        // every node on it in one parallel load (lane j <- depth j), so only
+        // the nodes that need a merge cost a dependent access.
+        uint64_t pmax = kInfPrio;
+        if (lane < levels) pmax = node_max(h, (p >> (levels - lane)) - 1);
+        for (int b = levels - 1; b >= 1; --b) prefetch_node(h, (p >> b) - 1, lane);  // the nodes themselves
+        for (int b = levels; b >= 1; --b) {
+            const uint32_t idx = (p >> b) - 1;
+            uint64_t fmin = __shfl_sync(kFull, F.prio, 0);
+            if (uniform_if(fmin < __shfl_sync(kFull, pmax, levels - b))) {
+                Entry<KW> M = ld_node(h, idx, lane);
+                Entry<KW> lo, hi;
+                merge2(M, F, lo, hi, lane);
+                st_node(h, idx, lane, lo);
+                F = hi;
+            }
         }
     }
     st_node(h, h.N, lane, F);
@@ -452,18 +447,19 @@ __device__ bool heap_push(WarpHeap<KW>& h, Entry<KW> x, uint32_t m, int lane) {
     if (m == 0) return true;
     x = sort32(x, lane);
     Entry<KW> lo, hi;
-    merge2(h.part, x, lo, hi, lane);
+    merge2(ld_part(h, lane), x, lo, hi, lane);
     const uint32_t tot = h.pc + m;
     if (tot < 32) {
-        h.part = lo;
+        st_part(h, lane, lo);
         h.pc = tot;
+        __syncwarp();
         return true;
     }
     // The largest 32 form a new node; the smallest stay in the partial buffer,
     // where the next pop sees them first.
     const uint32_t off = tot - 32;
     Entry<KW> node = pick(lo, hi, (int)off + lane);
-    h.part = (uint32_t)lane < off ? lo : inf_entry<KW>();
+    st_part(h, lane, (uint32_t)lane < off ? lo : inf_entry<KW>());
     h.pc = off;
     return heap_insert_node(h, node, lane);
 }
@@ -489,9 +485,8 @@ constexpr uint32_t kNoPage = 0xffffffffu;
 template <int KW> struct Buckets {
     Entry<KW>* pages;  // P pages of 32 entries (global memory)
     uint32_t* link;    // the page below each page in its bucket's stack (global memory)
-    uint32_t* fstack;  // pages freed while the register cache was full (global memory)
     uint32_t* upd;     // per-bucket scratch of a push (64 words, shared memory)
-    uint32_t* state;   // saved state of a suspended search (global memory)
+    uint32_t fs_off;   // link + fs_off: pages freed while the register cache was full
     uint32_t P;        // pages (0 = buckets off)
     uint32_t bump;     // pages >= bump were never used (warp-uniform)
     uint32_t nfs;      // entries on fstack (warp-uniform)
@@ -521,12 +516,12 @@ template <int KW> __device__ __forceinline__ uint32_t bq_min_f(const Buckets<KW>
     return q.lo + (uint32_t)(__ffs(rot) - 1);
 }
 
-template <int KW> __device__ __forceinline__ uint64_t open_min(const WarpHeap<KW>& h, const Buckets<KW>& q) {
-    const uint64_t hm = heap_min(h);
-    if (!q.P) return hm;
+// Least f over a warp's open list (kInf when it is empty).
+template <int KW> __device__ __forceinline__ uint32_t open_minf(const WarpHeap<KW>& h, const Buckets<KW>& q) {
+    const uint32_t hf = prio_f(heap_min(h));
+    if (!q.P) return hf;
     const uint32_t bf = bq_min_f(q);
-    const uint64_t bp = bf == kInf ? kInfPrio : ((uint64_t)bf << 32);
-    return hm < bp ? hm : bp;
+    return hf < bf ? hf : bf;
 }
 
 // Returns a freed page to the cache, or to the global stack when it is full.
@@ -535,7 +530,7 @@ template <int KW> __device__ __forceinline__ void bq_free(Buckets<KW>& q, uint32
         if ((uint32_t)lane == q.fc) q.cache = page;
         q.fc += 1;
     } else {
-        if (lane == 0) __stcg(q.fstack + q.nfs, page);
+        if (lane == 0) __stcg(q.link + q.fs_off + q.nfs, page);
         q.nfs += 1;
     }
 }
@@ -549,15 +544,8 @@ __device__ bool open_push(WarpHeap<KW>& h, Buckets<KW>& q, Entry<KW> x, uint32_t
     bool placed = false;
     if (q.P) {
         const uint32_t f = prio_f(x.prio);
-        if (!__any_sync(kFull, q.head != kNoPage)) {  // empty: the window starts at the least f
-            uint32_t mf = valid ? f : kInf;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const uint32_t t = __shfl_xor_sync(kFull, mf, o);
-                mf = t < mf ? t : mf;
-            }
-            q.lo = mf;
-        }
+        if (!__any_sync(kFull, q.head != kNoPage))  // empty: the window starts at the least f
+            q.lo = __reduce_min_sync(kFull, valid ? f : kInf);
         const bool inwin = valid && f >= q.lo && f - q.lo < 32u;
         const uint32_t b = f & 31u;
         const uint32_t lt = (1u << lane) - 1u;
@@ -579,7 +567,7 @@ __device__ bool open_push(WarpHeap<KW>& h, Buckets<KW>& q, Entry<KW> x, uint32_t
             if (leader && need && idx < avail) {
                 if (idx < q.fc) page = cached;
                 else if (idx < q.fc + fresh) page = q.bump + (idx - q.fc);
-                else page = __ldcg(q.fstack + q.nfs - 1 - (idx - q.fc - fresh));
+                else page = __ldcg(q.link + q.fs_off + q.nfs - 1 - (idx - q.fc - fresh));
             }
         }
         {
@@ -642,9 +630,9 @@ __device__ uint32_t open_pop(WarpHeap<KW>& h, Buckets<KW>& q, uint32_t E, uint64
         const uint32_t bf = bq_min_f(q);
         const uint64_t hm = heap_min(h);
         const uint64_t bp = bf == kInf ? kInfPrio : ((uint64_t)bf << 32);
-        if ((hm < bp ? hm : bp) >= lim) break;
+        if (uniform_if((hm < bp ? hm : bp) >= lim)) break;
         const uint32_t i = (uint32_t)lane - taken;  // this lane's index among the new ones
-        if (hm < bp) {  // the heap holds lower f: take its entries below the buckets' f
+        if (uniform_if(hm < bp)) {  // the heap holds lower f: take its entries below the buckets' f
             Entry<KW> e;
             const uint32_t c = heap_pop(h, E - taken, bp < lim ? bp : lim, e, lane);
             const Entry<KW> sh = shfl_idx(e, (lane - (int)taken) & 31);
@@ -653,7 +641,7 @@ __device__ uint32_t open_pop(WarpHeap<KW>& h, Buckets<KW>& q, uint32_t E, uint64
             if (c == 0) break;
         } else {
             const int bl = (int)(bf & 31u);
-            const uint32_t hd = __shfl_sync(kFull, q.head, bl), hc = __shfl_sync(kFull, q.hcnt, bl);
+            const uint32_t hd = __shfl_sync(kFull, q.head, bl), hc = uniform(__shfl_sync(kFull, q.hcnt, bl));
             const uint32_t k = E - taken < hc ? E - taken : hc;
             // The page's entries and, when it empties, its link load together.
             const uint32_t nx = hc == k ? __ldcg(q.link + hd) : kNoPage;
@@ -678,27 +666,27 @@ __device__ uint32_t open_pop(WarpHeap<KW>& h, Buckets<KW>& q, uint32_t E, uint64
 // The bucket state of a suspended search stays beside its pages: lane l
 // saves its bucket's head page and count and its cached free page; lane 0
 // the window start, the never-used and free-stack counts and the cache size.
-template <int KW> __device__ __forceinline__ void bq_save(const Buckets<KW>& q, int lane) {
+template <int KW> __device__ __forceinline__ void bq_save(const Buckets<KW>& q, uint32_t* state, int lane) {
     if (!q.P) return;
-    __stcg(q.state + lane, q.head);
-    __stcg(q.state + 32 + lane, q.hcnt);
-    __stcg(q.state + 64 + lane, q.cache);
+    __stcg(state + lane, q.head);
+    __stcg(state + 32 + lane, q.hcnt);
+    __stcg(state + 64 + lane, q.cache);
     if (lane == 0) {
-        __stcg(q.state + 96, q.lo);
-        __stcg(q.state + 97, q.bump);
-        __stcg(q.state + 98, q.nfs);
-        __stcg(q.state + 99, q.fc);
+        __stcg(state + 96, q.lo);
+        __stcg(state + 97, q.bump);
+        __stcg(state + 98, q.nfs);
+        __stcg(state + 99, q.fc);
     }
 }
-template <int KW> __device__ __forceinline__ void bq_restore(Buckets<KW>& q, int lane) {
+template <int KW> __device__ __forceinline__ void bq_restore(Buckets<KW>& q, const uint32_t* state, int lane) {
     if (!q.P) return;
-    q.head = __ldcg(q.state + lane);
-    q.hcnt = __ldcg(q.state + 32 + lane);
-    q.cache = __ldcg(q.state + 64 + lane);
-    q.lo = __ldcg(q.state + 96);
-    q.bump = __ldcg(q.state + 97);
-    q.nfs = __ldcg(q.state + 98);
-    q.fc = __ldcg(q.state + 99);
+    q.head = __ldcg(state + lane);
+    q.hcnt = __ldcg(state + 32 + lane);
+    q.cache = __ldcg(state + 64 + lane);
+    q.lo = uniform(__ldcg(state + 96));
+    q.bump = uniform(__ldcg(state + 97));
+    q.nfs = uniform(__ldcg(state + 98));
+    q.fc = uniform(__ldcg(state + 99));
 }
 
 // ---------------------------------------------------------------------------
@@ -708,11 +696,10 @@ template <int KW> __device__ __forceinline__ void bq_restore(Buckets<KW>& q, int
 // (fancy_hashmap.h:32-81, 155-167) as one atomic per successor.
 // ---------------------------------------------------------------------------
 
-// Claim protocol shared by the tables.  claim_first / claim_probe return
-//   -1 full, 2 home slot taken by another key (claim_probe walks on),
-//   0 found / 1 claimed, with `old` the value word before this update (done),
-//   4 found / 5 claimed, with the value still to be lowered by min_at.
-constexpr int kClNeedMin = 4;
+// Claims come in two steps: claim_begin issues the home slot's atomic,
+// claim_end resolves it -- probing on when the slot holds another key,
+// lowering the value of a known key -- and returns -1 full, 0 found or
+// 1 claimed, with `old` the value word before this update.
 
 __device__ __forceinline__ void cas128(unsigned long long* addr, uint64_t c0, uint64_t c1,
                                        uint64_t n0, uint64_t n1, uint64_t& o0, uint64_t& o1) {
@@ -737,42 +724,11 @@ struct HashTab64 {
     uint32_t max_probe;
 };
 
-__device__ __forceinline__ int tab_claim_at(const HashTab64& t, uint64_t i, uint64_t key, uint64_t val,
-                                            uint64_t& old) {
-    uint64_t o0, o1;
-    cas128(t.s + 2 * i, kEmpty, kEmpty, key, val, o0, o1);
-    if (o0 == kEmpty && o1 == kEmpty) {
-        old = kEmpty;
-        return 1;
-    }
-    if (o0 != key) return 2;
-    old = o1;
-    return o1 > val ? kClNeedMin : 0;
-}
-__device__ __forceinline__ int tab_claim_first(const HashTab64& t, uint64_t key, uint64_t val, uint64_t& slot,
-                                               uint64_t& old) {
-    const uint64_t i = mix64(key) & t.mask;
-    slot = 2 * i;
-    return tab_claim_at(t, i, key, val, old);
-}
-__device__ __forceinline__ int tab_claim_probe(const HashTab64& t, uint64_t key, uint64_t val, uint64_t& slot,
-                                               uint64_t& old) {
-    uint64_t i = slot / 2;
-    for (uint32_t p = 1; p < t.max_probe; ++p) {
-        i = (i + 1) & t.mask;
-        const int r = tab_claim_at(t, i, key, val, old);
-        if (r != 2) {
-            slot = 2 * i;
-            return r;
-        }
-    }
-    return -1;
-}
 // Lowers the value of a found key to `val` unless it is already <= val;
 // `seen` is the value the claim read.  Returns the value before the update.
 // Values only fall, so every failed exchange is followed by a strictly lower
 // value; the retry bound is far beyond the number of concurrent updaters.
-__device__ __forceinline__ uint64_t tab_min_at(const HashTab64& t, uint64_t slot, uint64_t key, uint64_t val,
+__device__ __forceinline__ uint64_t tab_min_at(const HashTab64& t, uint32_t slot, uint64_t key, uint64_t val,
                                                uint64_t seen) {
     uint64_t cur = seen;
     for (uint32_t r = 0; cur > val && r < 4096; ++r) {
@@ -783,28 +739,39 @@ __device__ __forceinline__ uint64_t tab_min_at(const HashTab64& t, uint64_t slot
     }
     return cur;
 }
+__device__ __forceinline__ void tab_claim_begin(const HashTab64& t, uint64_t key, uint64_t val, uint32_t& slot,
+                                                uint64_t& o0, uint64_t& o1) {
+    slot = 2 * (uint32_t)(mix64(key) & t.mask);
+    cas128(t.s + slot, kEmpty, kEmpty, key, val, o0, o1);
+}
+// (o0, o1): what claim_begin's exchange returned; o1 becomes the value before.
+__device__ __forceinline__ int tab_claim_end(const HashTab64& t, uint64_t key, uint64_t val, uint32_t& slot,
+                                             uint64_t o0, uint64_t& o1) {
+    for (uint32_t p = 1;; ++p) {
+        if (o0 == kEmpty && o1 == kEmpty) return 1;
+        if (o0 == key) {
+            if (o1 > val) o1 = tab_min_at(t, slot, key, val, o1);
+            return 0;
+        }
+        if (p >= t.max_probe) return -1;
+        slot = 2 * ((slot / 2 + 1) & (uint32_t)t.mask);
+        cas128(t.s + slot, kEmpty, kEmpty, key, val, o0, o1);
+    }
+}
 // Returns 1 when the key was newly claimed, 0 when found, -1 when full.
 __device__ __forceinline__ int tab_insert(const HashTab64& t, uint64_t key, uint64_t val, uint64_t& old,
-                                          uint64_t& slot) {
-    int r = tab_claim_first(t, key, val, slot, old);
-    if (r == 2) r = tab_claim_probe(t, key, val, slot, old);
-    if (r == kClNeedMin) {
-        old = tab_min_at(t, slot, key, val, old);
-        r = 0;
-    }
-    return r;
+                                          uint32_t& slot) {
+    uint64_t o0;
+    tab_claim_begin(t, key, val, slot, o0, old);
+    return tab_claim_end(t, key, val, slot, o0, old);
 }
 
-// Two-step lookup: look_begin issues the home-slot load, look_end resolves
-// it (probing on when the home slot holds another key), so the load can be in
-// flight while other memory work is issued.
-struct Look64 {
-    unsigned long long k, v;
-};
-__device__ __forceinline__ Look64 tab_look_begin(const HashTab64& t, uint64_t key) {
+// Issues the home-slot load of a lookup (key and value in one 16-byte load).
+__device__ __forceinline__ void tab_look_begin(const HashTab64& t, uint64_t key, uint64_t& k, uint64_t& v) {
     const uint64_t i = mix64(key) & t.mask;
     const ulonglong2 kv = __ldcg(reinterpret_cast<const ulonglong2*>(t.s + 2 * i));
-    return Look64{kv.x, kv.y};
+    k = kv.x;
+    v = kv.y;
 }
 
 __device__ __forceinline__ uint64_t tab_get(const HashTab64& t, uint64_t key) {
@@ -832,22 +799,31 @@ __device__ __forceinline__ uint64_t hash128(uint64_t k0, uint64_t k1) {
     return mix64(k0 ^ mix64(k1 + 0x9e3779b97f4a7c15ull));
 }
 
-__device__ __forceinline__ int tab_insert(const HashTab128& t, uint64_t k0, uint64_t k1,
-                                          uint64_t val, uint64_t& old, uint64_t& slot) {
-    uint64_t i = hash128(k0, k1) & t.mask;
-    for (uint32_t p = 0; p < t.max_probe; ++p) {
-        unsigned long long* ks = t.s + 4 * i;
-        uint64_t o0, o1;
-        cas128(ks, kEmpty, kEmpty, k0, k1, o0, o1);
-        int claimed = (o0 == kEmpty && o1 == kEmpty);
+__device__ __forceinline__ void tab_claim_begin(const HashTab128& t, uint64_t k0, uint64_t k1, uint32_t& slot,
+                                                uint64_t& o0, uint64_t& o1) {
+    slot = 4 * (uint32_t)(hash128(k0, k1) & t.mask);
+    cas128(t.s + slot, kEmpty, kEmpty, k0, k1, o0, o1);
+}
+// (o0, o1): the key words claim_begin's exchange returned; o1 becomes the
+// value before.  The value word beside the key is lowered with atomicMin.
+__device__ __forceinline__ int tab_claim_end(const HashTab128& t, uint64_t k0, uint64_t k1, uint64_t val,
+                                             uint32_t& slot, uint64_t o0, uint64_t& o1) {
+    for (uint32_t p = 1;; ++p) {
+        const int claimed = (o0 == kEmpty && o1 == kEmpty);
         if (claimed || (o0 == k0 && o1 == k1)) {
-            old = atomicMin(ks + 2, val);
-            slot = 4 * i;
+            o1 = atomicMin(t.s + slot + 2, (unsigned long long)val);
             return claimed;
         }
-        i = (i + 1) & t.mask;
+        if (p >= t.max_probe) return -1;
+        slot = 4 * ((slot / 4 + 1) & (uint32_t)t.mask);
+        cas128(t.s + slot, kEmpty, kEmpty, k0, k1, o0, o1);
     }
-    return -1;
+}
+__device__ __forceinline__ int tab_insert(const HashTab128& t, uint64_t k0, uint64_t k1,
+                                          uint64_t val, uint64_t& old, uint32_t& slot) {
+    uint64_t o0;
+    tab_claim_begin(t, k0, k1, slot, o0, old);
+    return tab_claim_end(t, k0, k1, val, slot, o0, old);
 }
 
 __device__ __forceinline__ uint64_t tab_get(const HashTab128& t, uint64_t k0, uint64_t k1) {
@@ -863,37 +839,18 @@ __device__ __forceinline__ uint64_t tab_get(const HashTab128& t, uint64_t k0, ui
     return kEmpty;
 }
 
+// Issues the home slot's reads of a lookup: the key pair (one 16-byte atomic)
+// and the value word.
+__device__ __forceinline__ void tab_look_begin(const HashTab128& t, uint64_t k0, uint64_t k1, uint64_t& o0,
+                                               uint64_t& o1, uint64_t& v) {
+    unsigned long long* ks = t.s + 4 * (hash128(k0, k1) & t.mask);
+    cas128(ks, kEmpty, kEmpty, kEmpty, kEmpty, o0, o1);
+    v = __ldcg(ks + 2);
+}
+
 // Dense table for grids: the cell index is the slot (a perfect hash).
 struct DenseTab {
     unsigned long long* v;
 };
-
-// 128-bit keys: the key pair is claimed with a 16-byte compare-and-swap, the
-// value word beside it is lowered with atomicMin.
-__device__ __forceinline__ int tab_claim_first(const HashTab128& t, uint64_t k0, uint64_t k1, uint64_t& slot) {
-    const uint64_t i = hash128(k0, k1) & t.mask;
-    slot = 4 * i;
-    uint64_t o0, o1;
-    cas128(t.s + 4 * i, kEmpty, kEmpty, k0, k1, o0, o1);
-    if (o0 == kEmpty && o1 == kEmpty) return kClNeedMin | 1;
-    return (o0 == k0 && o1 == k1) ? kClNeedMin : 2;
-}
-__device__ __forceinline__ int tab_claim_probe(const HashTab128& t, uint64_t k0, uint64_t k1, uint64_t& slot) {
-    uint64_t i = slot / 4;
-    for (uint32_t p = 1; p < t.max_probe; ++p) {
-        i = (i + 1) & t.mask;
-        uint64_t o0, o1;
-        cas128(t.s + 4 * i, kEmpty, kEmpty, k0, k1, o0, o1);
-        const int claimed = (o0 == kEmpty && o1 == kEmpty);
-        if (claimed || (o0 == k0 && o1 == k1)) {
-            slot = 4 * i;
-            return kClNeedMin | claimed;
-        }
-    }
-    return -1;
-}
-__device__ __forceinline__ uint64_t tab_min_at(const HashTab128& t, uint64_t slot, uint64_t val) {
-    return atomicMin(t.s + slot + 2, val);
-}
 
 }  // namespace gastar

@@ -44,7 +44,7 @@ constexpr uint32_t kCuts = 16;  // cut slots in the ring (> 3 * kCutLag + 2)
 // iteration i - kStageRing, must be no later than that.
 static_assert(kStageRing >= kCutLag + 2, "a stage buffer must be consumed before it is reused");
 
-constexpr uint32_t kSlotsHost = 4;
+constexpr uint32_t kMaxWarps = 16;  // warps of the largest block
 
 // Plain engine: iteration from which a puzzle search with the automatic
 // expansion width pops twice as many entries per warp-heap.
@@ -136,15 +136,18 @@ inline __host__ __device__ size_t bucket_area_bytes(uint32_t heaps, uint32_t pag
     return (size_t)heaps * pages * (32 * (size_t)entry_bytes + 8) + (size_t)heaps * kBucketStateWords * 4;
 }
 
-// Per-iteration state of a one-block team (shared memory); iteration t uses
-// slot t % kSlots.
+// Per-iteration record of a block (shared memory): 32-bit fields, whose
+// shared-memory atomics are single instructions.  A one-block team keeps
+// kSlots of them, iteration t using slot t % kSlots.
 struct alignas(16) TeamSlot {
-    unsigned long long minprio;   // min priority over the team's heaps after the push phase
-    unsigned long long minstage;  // min priority of the entries staged in the pop/expand phase
-    uint32_t count;               // entries staged in the pop/expand phase
-    uint32_t best;                // goal costs found in the pop/expand phase
-    uint32_t err;                 // first error raised in the iteration
-    uint32_t pad;
+    uint32_t count;     // entries staged in the pop/expand phase
+    uint32_t minstage;  // least f of the entries staged
+    uint32_t best;      // goal costs found in the pop/expand phase
+    uint32_t err;       // first error raised in the pop/expand phase
+    uint32_t claims;    // table slots claimed
+    uint32_t exps;      // entries expanded
+    uint32_t minheap;   // least f over the heaps after the push phase
+    uint32_t perr;      // error raised in the push phase
 };
 constexpr uint32_t kSlots = 4;
 
@@ -154,11 +157,11 @@ constexpr uint32_t kSlots = 4;
 // slot with atomics in the same few hundred nanoseconds: each of them has its
 // own 128-byte line, so those atomics queue at different L2 slices.
 struct alignas(128) CutSlot {
-    unsigned long long minprio;  // min priority over the team's heaps
+    uint32_t minf;               // least f over the team's open lists
     uint32_t best;               // goal costs found in the iteration before
     uint32_t lossy;              // entries were lost (table or heap full, cost range)
     uint32_t err;                // budget or timeout
-    uint32_t pad0[27];
+    uint32_t pad0[28];
     unsigned long long claims;   // table slots the blocks claimed since their last cut
     uint32_t pad1[30];
     unsigned long long exps;     // expansions since the blocks' last cut
@@ -184,7 +187,7 @@ inline void team_ctl_init(TeamCtl& t) {
     t.inst = 0;
     for (auto& p : t.pad) p = 0;
     for (auto& c : t.cut) {
-        c.minprio = ~0ull;
+        c.minf = 0xffffffffu;
         c.claims = c.exps = 0;
         c.best = 0xffffffffu;
         c.lossy = c.err = c.count = 0;

@@ -120,10 +120,8 @@ struct PluginDom {
     static constexpr bool kDense = false;
     static constexpr uint32_t kRootCode = 0xffffffffu;
     static constexpr bool kParentBySlot = true;  // no inverse moves: parents by table slot
-    struct Look {};                              // the own-slot lookup precedes the probes
     using KeyT = PlainKey<KW>;
     using Tab = HashTabLock<KW>;
-    using Pre = int;
 
     struct Ctx {
         KeyT goal, start;
@@ -188,31 +186,25 @@ struct PluginDom {
     }
     static __device__ __forceinline__ uint32_t code(int, uint32_t self) { return self; }
     static __device__ __forceinline__ int insert(const Tab& t, const KeyT& k, uint64_t v, uint64_t& old,
-                                                 uint64_t& slot) {
+                                                 uint32_t& slot) {
         uint64_t i;
         const int r = lock_claim<KW>(t, k, i);
         if (r < 0) return r;
         old = atomicMin(t.s + i * Tab::SW + 1 + KW, v);
-        slot = i;
+        slot = (uint32_t)i;
         return r;
     }
-    static __device__ __forceinline__ int claim_first(const Tab& t, const KeyT& k, uint64_t, uint64_t& slot,
-                                                      uint64_t&) {
-        const int r = lock_claim<KW>(t, k, slot);
-        return r < 0 ? r : kClNeedMin | r;
-    }
-    static __device__ __forceinline__ int claim_probe(const Tab&, const KeyT&, uint64_t, uint64_t&, uint64_t&) {
-        return -1;
-    }
-    static __device__ __forceinline__ uint64_t min_at(const Tab& t, uint64_t slot, const KeyT&, uint64_t v,
-                                                      uint64_t) {
-        return atomicMin(t.s + slot * Tab::SW + 1 + KW, v);
+    // The whole claim resolves in claim_end: lock_claim may wait for a writer.
+    static __device__ __forceinline__ void claim_begin(const Tab&, const KeyT&, uint64_t, uint32_t&, uint64_t&,
+                                                       uint64_t&) {}
+    static __device__ __forceinline__ int claim_end(const Tab& t, const KeyT& k, uint64_t v, uint32_t& slot, uint64_t,
+                                                    uint64_t& old) {
+        return insert(t, k, v, old, slot);
     }
     static __device__ __forceinline__ bool is_goal(const Ctx& c, const KeyT& k) { return k == c.goal; }
     static __device__ __forceinline__ bool is_start(const Ctx& c, const KeyT& k) { return k == c.start; }
-    static __device__ __forceinline__ Pre prepare(const Ctx&, const KeyT&) { return 0; }
-    static __device__ __forceinline__ bool succ(const Ctx&, const KeyT& k, Pre, int m, uint32_t, uint32_t g,
-                                                uint32_t, KeyT& nk, uint32_t& ng, uint32_t& nh) {
+    static __device__ __forceinline__ bool succ(const Ctx&, const KeyT& k, int m, uint32_t g, uint32_t, KeyT& nk,
+                                                uint32_t& ng, uint32_t& nh) {
         const T src = from_key(k);
         T dst = src;
         bool ex = false;
@@ -235,12 +227,16 @@ struct PluginDom {
 
 // One plugin instance on every block of the launch (cooperative when the
 // team has more than one block).
-template <class D> __global__ void __launch_bounds__(256, 1) plugin_search_kernel(LaunchParams P) {
-    __shared__ CtaShared sm;
-    __shared__ typename D::Ctx ctx;
-    if (threadIdx.x == 0) sm.desc = P.insts[0];
+template <class D> __global__ void __launch_bounds__(256, 1) plugin_search_kernel(const __grid_constant__ LaunchParams P) {
+    if (threadIdx.x == 0) {
+        cta().desc = P.insts[0];
+        cta().slice = 0;
+    }
     __syncthreads();
-    run_instance<D>(P, sm.desc, sm, ctx, TeamRef{P.team_ctas, P.team_ctas > 1 ? blockIdx.x : 0u, P.team, P.stage});
+    if (P.team_ctas > 1)
+        run_instance<D, 256, TEAM_RING>(P, TeamRef{P.team_ctas, blockIdx.x, P.team, P.stage});
+    else
+        run_instance<D, 256, TEAM_BLOCK>(P, TeamRef{1, 0, nullptr, nullptr});
 }
 
 template <class D>

@@ -5,10 +5,10 @@
 // iteration is
 //   pop    : every warp pops up to `ew` best entries (one per lane), drops
 //            stale ones (table g lower than the entry's g) and goal states;
-//   expand : every lane generates the successors of its entry, computes g and
-//            an incrementally updated h, and does one insert-or-min on the
-//            duplicate-detection table per successor; improved successors go
-//            to the block's stage area;
+//   expand : a group of lanes per entry, one lane per move, generates the
+//            successors, computes g and an incrementally updated h, and does
+//            one insert-or-min on the duplicate-detection table per
+//            successor; improved successors go to the block's stage area;
 //   push   : one-block teams deal their stage chunks round-robin (rotating
 //            offset) to their warps after a block barrier; in a multi-block
 //            team block c pushes the stage region of block (c + i) mod blocks
@@ -44,7 +44,6 @@ template <int N> struct SlidingDom {
     static constexpr int C = N * N;
     using KeyT = std::conditional_t<KW == 1, uint64_t, unsigned __int128>;
     using Tab = std::conditional_t<KW == 1, HashTab64, HashTab128>;
-    using Pre = int;  // blank cell
 
     struct Ctx {
         KeyT goal, start;
@@ -122,56 +121,51 @@ template <int N> struct SlidingDom {
     // Parents are recorded by move code; the root's code is kRootMove.
     static constexpr uint32_t kRootCode = kRootMove;
     static constexpr bool kParentBySlot = false;
-    struct Look {
-        uint64_t k, v;
-    };
-    static __device__ __forceinline__ Look look_begin(const Tab& t, KeyT k) {
+    // Two-step lookup of an entry's own value: look_begin issues the home
+    // slot's reads (key words k0, k1 and value v), look_end resolves them,
+    // probing on when the home slot holds another key.
+    static __device__ __forceinline__ void look_begin(const Tab& t, KeyT k, uint64_t& k0, uint64_t& k1, uint64_t& v) {
         if constexpr (KW == 1) {
-            const Look64 l = tab_look_begin(t, k);
-            return Look{l.k, l.v};
+            k1 = 0;
+            tab_look_begin(t, k, k0, v);
         } else {
-            return Look{0, 0};
+            tab_look_begin(t, uint64_t(k), uint64_t(k >> 64), k0, k1, v);
         }
     }
-    static __device__ __forceinline__ uint64_t look_end(const Tab& t, KeyT k, const Look& l) {
-        if constexpr (KW == 1) {
-            if (l.k == k) return l.v;
-            if (l.k == kEmpty) return kEmpty;
-        }
-        return get(t, k);
+    static __device__ __forceinline__ uint64_t look_end(const Tab& t, KeyT k, uint64_t k0, uint64_t k1, uint64_t v) {
+        bool empty = k0 == kEmpty;
+        if constexpr (KW == 2) empty = empty && k1 == kEmpty;
+        if (empty) return kEmpty;
+        const KeyT seen = desc_key(k0, k1);
+        return seen == k ? v : get(t, k);
     }
-    static __device__ __forceinline__ uint64_t get_self(const Tab& t, KeyT k, uint32_t&) { return get(t, k); }
     static __device__ __forceinline__ uint32_t code(int m, uint32_t) { return (uint32_t)m; }
     static __device__ __forceinline__ int insert(const Tab& t, KeyT k, uint64_t v, uint64_t& old,
-                                                 uint64_t& slot) {
+                                                 uint32_t& slot) {
         if constexpr (KW == 1) return tab_insert(t, k, v, old, slot);
         else return tab_insert(t, uint64_t(k), uint64_t(k >> 64), v, old, slot);
     }
     static constexpr bool kDense = false;
-    static __device__ __forceinline__ int claim_first(const Tab& t, KeyT k, uint64_t v, uint64_t& slot,
-                                                      uint64_t& old) {
-        if constexpr (KW == 1) return tab_claim_first(t, k, v, slot, old);
-        else return tab_claim_first(t, uint64_t(k), uint64_t(k >> 64), slot);
+    // Two-step claim: claim_begin issues the home slot's compare-and-swap (the
+    // words it returned in k0, k1), claim_end resolves it (see tab_claim_end).
+    static __device__ __forceinline__ void claim_begin(const Tab& t, KeyT k, uint64_t v, uint32_t& slot, uint64_t& k0,
+                                                       uint64_t& k1) {
+        if constexpr (KW == 1) tab_claim_begin(t, k, v, slot, k0, k1);
+        else tab_claim_begin(t, uint64_t(k), uint64_t(k >> 64), slot, k0, k1);
     }
-    static __device__ __forceinline__ int claim_probe(const Tab& t, KeyT k, uint64_t v, uint64_t& slot,
-                                                      uint64_t& old) {
-        if constexpr (KW == 1) return tab_claim_probe(t, k, v, slot, old);
-        else return tab_claim_probe(t, uint64_t(k), uint64_t(k >> 64), slot);
-    }
-    static __device__ __forceinline__ uint64_t min_at(const Tab& t, uint64_t slot, KeyT k, uint64_t v,
-                                                      uint64_t seen) {
-        if constexpr (KW == 1) return tab_min_at(t, slot, k, v, seen);
-        else return tab_min_at(t, slot, v);
+    static __device__ __forceinline__ int claim_end(const Tab& t, KeyT k, uint64_t v, uint32_t& slot, uint64_t k0,
+                                                    uint64_t& k1) {
+        if constexpr (KW == 1) return tab_claim_end(t, k, v, slot, k0, k1);
+        else return tab_claim_end(t, uint64_t(k), uint64_t(k >> 64), v, slot, k0, k1);
     }
     static __device__ __forceinline__ bool is_goal(const Ctx& c, KeyT k) { return k == c.goal; }
     static __device__ __forceinline__ bool is_start(const Ctx& c, KeyT k) { return k == c.start; }
-    static __device__ __forceinline__ Pre prepare(const Ctx&, KeyT k) { return blank_of(k); }
+    // Whether move m leads straight back to the parent reached with move pm.
+    static __device__ __forceinline__ bool is_back(int m, uint32_t pm) { return (uint32_t)(m ^ 1) == pm; }
 
-    static __device__ __forceinline__ bool succ(const Ctx& c, KeyT k, Pre p, int m, uint32_t pm,
-                                                uint32_t g, uint32_t h, KeyT& nk, uint32_t& ng,
-                                                uint32_t& nh) {
-        if ((uint32_t)(m ^ 1) == pm) return false;  // straight back to the parent
-        const int r = p / N, col = p % N;
+    static __device__ __forceinline__ bool succ(const Ctx& c, KeyT k, int m, uint32_t g, uint32_t h, KeyT& nk,
+                                                uint32_t& ng, uint32_t& nh) {
+        const int p = blank_of(k), r = p / N, col = p % N;
         int q;
         if (m == 0) {
             if (r >= N - 1) return false;
@@ -209,23 +203,29 @@ template <int N> struct SlidingDom {
 // weight; weight 0 is impassable.  The duplicate-detection table is a dense
 // value array indexed by cell.
 // ---------------------------------------------------------------------------
+// GridDom::dx(m) + 1 and GridDom::dy(m) + 1 in bits 2m..2m+1.
+constexpr uint32_t kGridDxPack = 2u | 0u << 2 | 1u << 4 | 1u << 6 | 2u << 8 | 2u << 10 | 0u << 12 | 0u << 14;
+constexpr uint32_t kGridDyPack = 1u | 1u << 2 | 2u << 4 | 0u << 6 | 2u << 8 | 0u << 10 | 2u << 12 | 0u << 14;
+
 struct GridDom {
     static constexpr int KW = 1;
     static constexpr int MAXN = 8;
     using KeyT = uint64_t;
     using Tab = DenseTab;
-    struct Pre {
-        int x, y;
-        uint64_t wts;  // byte m: weight of the cell move m enters (0 = obstacle or off the board)
-    };
+    // Key: cell index | x << 32 | y << 48 (sides are at most 65535); the table
+    // is indexed by the cell.
+    static __host__ __device__ __forceinline__ KeyT make_key(uint32_t cell, uint32_t x, uint32_t y) {
+        return (KeyT)cell | (KeyT)x << 32 | (KeyT)y << 48;
+    }
 
     struct Ctx {
         const uint8_t* w;
-        uint32_t W, H, goal, start, gx, gy, minw, href;
+        KeyT start;
+        uint32_t W, H, goal, gx, gy, minw, href;
     };
 
-    static __device__ __forceinline__ int dx(int m) { return (m == 0 || m == 4 || m == 5) ? 1 : (m == 1 || m == 6 || m == 7) ? -1 : 0; }
-    static __device__ __forceinline__ int dy(int m) { return (m == 2 || m == 4 || m == 6) ? 1 : (m == 3 || m == 5 || m == 7) ? -1 : 0; }
+    static constexpr __host__ __device__ int dx(int m) { return (m == 0 || m == 4 || m == 5) ? 1 : (m == 1 || m == 6 || m == 7) ? -1 : 0; }
+    static constexpr __host__ __device__ int dy(int m) { return (m == 2 || m == 4 || m == 6) ? 1 : (m == 3 || m == 5 || m == 7) ? -1 : 0; }
     static __device__ __forceinline__ uint32_t inv(uint32_t m) { return m < 4 ? (m ^ 1) : 11 - m; }
 
     static __device__ __forceinline__ KeyT key_of(const Entry<1>& e) { return e.k[0]; }
@@ -237,7 +237,8 @@ struct GridDom {
             c.W = d.W;
             c.H = d.H;
             c.goal = (uint32_t)d.goal0;
-            c.start = (uint32_t)d.start0;
+            const uint32_t st = (uint32_t)d.start0;
+            c.start = make_key(st, st % d.W, st / d.W);
             c.gx = c.goal % d.W;
             c.gy = c.goal / d.W;
             c.minw = d.minw;
@@ -246,51 +247,25 @@ struct GridDom {
         __syncthreads();
     }
     static __device__ __forceinline__ Tab make_tab(const InstDesc& d) { return Tab{d.table}; }
-    static __device__ __forceinline__ uint64_t get(const Tab& t, KeyT k) { return __ldcg(t.v + k); }
+    static __device__ __forceinline__ uint64_t get(const Tab& t, KeyT k) { return __ldcg(t.v + (uint32_t)k); }
     static __device__ __forceinline__ uint32_t start_f(const Ctx&, const InstDesc& d) { return d.f0; }
     static constexpr uint32_t kRootCode = kRootMove;
     static constexpr bool kParentBySlot = false;
-    struct Look {
-        uint64_t v;
-    };
-    static __device__ __forceinline__ Look look_begin(const Tab& t, KeyT k) { return Look{__ldcg(t.v + k)}; }
-    static __device__ __forceinline__ uint64_t look_end(const Tab&, KeyT, const Look& l) { return l.v; }
-    static __device__ __forceinline__ uint64_t get_self(const Tab& t, KeyT k, uint32_t&) { return get(t, k); }
     static __device__ __forceinline__ uint32_t code(int m, uint32_t) { return (uint32_t)m; }
-    static __device__ __forceinline__ int insert(const Tab& t, KeyT k, uint64_t v, uint64_t& old,
-                                                 uint64_t& slot) {
-        old = atomicMin(t.v + k, v);
-        slot = k;
-        return old == kEmpty ? 1 : 0;
-    }
     static constexpr bool kDense = true;
     // The cell is the slot: one atomicMin claims and lowers it.
-    static __device__ __forceinline__ int claim_first(const Tab& t, KeyT k, uint64_t v, uint64_t& slot,
-                                                      uint64_t& old) {
-        slot = k;
-        old = atomicMin(t.v + k, v);
+    static __device__ __forceinline__ uint64_t lower(const Tab& t, KeyT k, uint64_t v) {
+        return atomicMin(t.v + (uint32_t)k, (unsigned long long)v);
+    }
+    static __device__ __forceinline__ int insert(const Tab& t, KeyT k, uint64_t v, uint64_t& old,
+                                                 uint32_t& slot) {
+        old = lower(t, k, v);
+        slot = (uint32_t)k;
         return old == kEmpty ? 1 : 0;
     }
-    static __device__ __forceinline__ int claim_probe(const Tab&, KeyT, uint64_t, uint64_t&, uint64_t&) {
-        return -1;
-    }
-    static __device__ __forceinline__ uint64_t min_at(const Tab& t, uint64_t slot, KeyT, uint64_t v, uint64_t) {
-        return atomicMin(t.v + slot, v);
-    }
-    static __device__ __forceinline__ bool is_goal(const Ctx& c, KeyT k) { return k == c.goal; }
-    static __device__ __forceinline__ bool is_start(const Ctx& c, KeyT k) { return k == c.start; }
-    // The eight neighbours' weights load together, before any successor
-    // needs one (every load is inside the board, whatever k holds).
-    static __device__ __forceinline__ Pre prepare(const Ctx& c, KeyT k) {
-        const uint32_t cell = (uint32_t)k;
-        Pre p{(int)(cell % c.W), (int)(cell / c.W), 0};
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const int nx = p.x + dx(m), ny = p.y + dy(m);
-            if (nx >= 0 && ny >= 0 && nx < (int)c.W && ny < (int)c.H)
-                p.wts |= (uint64_t)__ldg(c.w + (uint32_t)ny * c.W + (uint32_t)nx) << (8 * m);
-        }
-        return p;
+    static __device__ __forceinline__ bool is_goal(const Ctx& c, KeyT k) { return (uint32_t)k == c.goal; }
+    static __device__ __forceinline__ bool is_back(int m, uint32_t pm) {
+        return pm != kRootMove && (uint32_t)m == inv(pm);
     }
     static __device__ __forceinline__ uint32_t heur(const Ctx& c, int x, int y) {
         // 0: Chebyshev x min weight (admissible); 1: Manhattan (the reference's,
@@ -300,38 +275,30 @@ struct GridDom {
         if (c.href == 2) return 0;
         return (ax > ay ? ax : ay) * c.minw;
     }
-    static __device__ __forceinline__ bool succ(const Ctx& c, KeyT, Pre p, int m, uint32_t pm,
-                                                uint32_t g, uint32_t, KeyT& nk, uint32_t& ng,
-                                                uint32_t& nh) {
-        if (pm != kRootMove && (uint32_t)m == inv(pm)) return false;
-        const uint32_t wt = (uint32_t)(p.wts >> (8 * m)) & 0xffu;
-        if (!wt) return false;  // obstacle or off the board
-        const int nx = p.x + dx(m), ny = p.y + dy(m);
-        const uint32_t cell = (uint32_t)ny * c.W + (uint32_t)nx;
-        nk = cell;
-        ng = g + wt;
+    // The cell move m enters from k and its h; false off the board.
+    static __device__ __forceinline__ bool step(const Ctx& c, KeyT k, int m, KeyT& nk, uint32_t& nh) {
+        const int ddx = (int)((kGridDxPack >> (2 * m)) & 3u) - 1, ddy = (int)((kGridDyPack >> (2 * m)) & 3u) - 1;
+        const int nx = (int)(uint32_t)(k >> 32 & 0xffffu) + ddx, ny = (int)(uint32_t)(k >> 48) + ddy;
+        if ((uint32_t)nx >= c.W || (uint32_t)ny >= c.H) return false;
+        nk = make_key((uint32_t)k + (uint32_t)(ddy * (int)c.W + ddx), (uint32_t)nx, (uint32_t)ny);
         nh = heur(c, nx, ny);
         return true;
     }
-    static __device__ __forceinline__ KeyT parent(const Ctx& c, const Tab&, KeyT k, uint32_t m) {
-        return (KeyT)((int64_t)k - dx((int)m) - (int64_t)dy((int)m) * (int64_t)c.W);
-    }
+    static __device__ __forceinline__ uint32_t weight(const Ctx& c, KeyT k) { return __ldg(c.w + (uint32_t)k); }
 };
 
 // ---------------------------------------------------------------------------
 // Block-shared state.
 // ---------------------------------------------------------------------------
 struct CtaShared {
-    TeamSlot slot[kSlots];  // team slots of a one-block team
+    TeamSlot slot[kSlots];  // iteration records of a one-block team
     TeamSlot agg;           // this block's share of the current iteration (multi-block teams)
-    unsigned long long agg_minprio;  // this block's heaps' min after the previous push
-    unsigned long long cnt[5];       // expansions, stale, generated, pushes, claims of this block
-                                     // in this launch (added to the control block at exit)
-    unsigned long long pub[2];       // claims, expansions as of the last published cut
-    unsigned long long run[2];       // claims, expansions of the cuts tested so far
-    unsigned long long base[2];      // claims, expansions before this launch
-    unsigned long long t_start;      // search start on the device clock
-    uint32_t agg_err_prev;           // heap full in the previous push
+    uint32_t agg_minheap, agg_err_prev;  // this block's heaps' min f and error of the previous push
+    unsigned long long run[2];   // claims, expansions of the iterations tested so far
+    unsigned long long mine[2];  // claims, expansions of this block (multi-block teams)
+    unsigned long long base[2];  // claims, expansions before this launch
+    unsigned long long wcnt[kMaxWarps][3];  // per warp: stale, generated, pushed in this launch
+    unsigned long long t_start;  // search start on the device clock
     uint32_t dec_status, dec_best, dec_fmin, push_count;  // thread 0 -> block
     InstDesc desc;
     uint32_t inst, ok, slice, pad1;  // slice: iterations before suspending (0 = to the end)
@@ -345,12 +312,32 @@ struct CtaShared {
 
 extern __shared__ uint4 g_dyn_smem[];
 
+// The block's shared state.  A function-local variable rather than a reference
+// handed down: every access is then a shared-memory instruction instead of a
+// generic one, and costs no register for the address.
+__device__ __forceinline__ CtaShared& cta() {
+    __shared__ CtaShared s;
+    return s;
+}
+template <class D> __device__ __forceinline__ typename D::Ctx& shared_ctx() {  // plugins
+    __shared__ typename D::Ctx c;
+    return c;
+}
+__device__ __forceinline__ void slot_clear(TeamSlot& t) {
+    t.count = t.err = t.claims = t.exps = t.perr = 0;
+    t.minstage = t.best = t.minheap = kInf;
+}
+template <> __device__ __forceinline__ SlidingDom<3>::Ctx& shared_ctx<SlidingDom<3>>() { return cta().ctx.s3; }
+template <> __device__ __forceinline__ SlidingDom<4>::Ctx& shared_ctx<SlidingDom<4>>() { return cta().ctx.s4; }
+template <> __device__ __forceinline__ SlidingDom<5>::Ctx& shared_ctx<SlidingDom<5>>() { return cta().ctx.s5; }
+template <> __device__ __forceinline__ GridDom::Ctx& shared_ctx<GridDom>() { return cta().ctx.g; }
+
 // Barrier over the blocks of a multi-block team: one atomic arrival on a
 // counter that only grows, a poll until it reaches the end of this barrier's
 // range, a bounded wait (deadline on the device clock), and an abort flag so
 // that one block giving up releases the others.
-__device__ __forceinline__ bool team_sync_grid(TeamCtl* tc, uint32_t nctas, uint64_t timeout_ns,
-                                               CtaShared& sm) {
+__device__ __forceinline__ bool team_sync_grid(TeamCtl* tc, uint32_t nctas, uint64_t timeout_ns) {
+    CtaShared& sm = cta();
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t ok = 1;
@@ -472,89 +459,80 @@ struct TeamRef {
     void* stage;    // stage buffers of a multi-block team (device)
 };
 
-// Inclusive warp prefix sum.
-__device__ __forceinline__ uint32_t warp_incl_sum(uint32_t v, int lane) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(kFull, v, o);
-        if (lane >= o) v += t;
-    }
-    return v;
+// Lanes of a warp that expand one entry: a power of two, one lane per move
+// (domains with more than 32 moves take them 32 at a time).
+constexpr int lanes_per_entry(int maxn) {
+    int l = 1;
+    while (l < maxn && l < 32) l *= 2;
+    return l;
 }
-__device__ __forceinline__ uint64_t warp_min64(uint64_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const uint64_t t = __shfl_xor_sync(kFull, v, o);
-        v = t < v ? t : v;
-    }
-    return v;
+template <int LPE> __device__ constexpr uint32_t group_mask() {
+    return LPE == 32 ? 0xffffffffu : (1u << (LPE & 31)) - 1u;
 }
 
 
-template <class D>
-__device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc& d, CtaShared& sm,
-                                          typename D::Ctx& ctx, const TeamRef tm) {
+// How the blocks of a team work together.
+enum TeamKind : int { TEAM_BLOCK, TEAM_RING };
+
+template <class D, int MAXT, int TEAM>
+__device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef tm) {
     constexpr int KW = D::KW;
     constexpr int MAXN = D::MAXN;
+    constexpr bool multi = TEAM == TEAM_RING;
     using E = Entry<KW>;
     using KeyT = typename D::KeyT;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    const bool multi = tm.ctas > 1;
-    const uint32_t rank = tm.rank;
-    const uint32_t H = d.heaps;
-    TeamSlot* slots = sm.slot;  // one-block teams
-    const uint32_t ew_cap = d.ew_wide > d.ew ? d.ew_wide : d.ew;  // widest pop of the search
-    const size_t stage_cap = stage_entries_per_buffer(H, ew_cap, MAXN);
-    char* dyn = reinterpret_cast<char*>(g_dyn_smem);
-    E* const stage0 = multi ? reinterpret_cast<E*>(tm.stage) : reinterpret_cast<E*>(dyn);  // ring (multi)
-    E* const snodes_all = reinterpret_cast<E*>(dyn + (multi ? 0 : 2 * stage_cap * sizeof(E)));
-    InstCtl* ctl = d.ctl;
+    constexpr int LPE = lanes_per_entry(MAXN);  // lanes per entry: one per move
+    constexpr int EPR = 32 / LPE;               // entries per expansion round
+    // Rounds whose probes are in flight together (registers: 16-warp blocks
+    // have 128 per thread, and twice the warps to overlap).
+    constexpr int RB = KW == 1 && MAXT <= 256 ? 4 : 2;
+    CtaShared& sm = cta();
+    const InstDesc& d = sm.desc;
+    typename D::Ctx& ctx = shared_ctx<D>();
+    const int lane = threadIdx.x & 31, warp = (int)uniform(threadIdx.x >> 5), W = blockDim.x >> 5;
+    const uint32_t rank = multi ? tm.rank : 0u;
+    InstCtl* const ctl = d.ctl;
     const bool leader = rank == 0 && threadIdx.x == 0;
+    const uint32_t hid = rank * W + warp;
+    // One-block teams stage in shared memory (two buffers), multi-block teams
+    // in a global ring.
+    const uint32_t region_cap =
+        (uint32_t)stage_entries_per_buffer(W, d.ew_wide > d.ew ? d.ew_wide : d.ew, MAXN);  // widest pop of the search
+    E* const snodes_all = reinterpret_cast<E*>(g_dyn_smem) + (multi ? 0u : 2 * region_cap);
 
     auto tsync = [&]() -> bool {
-        if (!multi) {
-            __syncthreads();
-            return true;
-        }
-        return team_sync_grid(tm.ctl, tm.ctas, P.barrier_timeout_ns, sm);
+        if constexpr (multi) return team_sync_grid(tm.ctl, tm.ctas, P.barrier_timeout_ns);
+        __syncthreads();
+        return true;
     };
 
     D::load(ctx, d);
-    const typename D::Tab tab = D::make_tab(d);
 
     WarpHeap<KW> hp;
-    const uint32_t hid = rank * W + warp;
     hp.nodes = reinterpret_cast<E*>(d.heap_nodes) + (size_t)hid * (d.heap_cap + 1) * 32;
-    hp.sn = P.heap_snodes ? P.heap_snodes : kHeapSmemNodes;
-    hp.snodes = snodes_all + (size_t)warp * (hp.sn - 1) * 32;
-    hp.hdr = d.heap_hdr + 2 * hid;
-    hp.cap = d.heap_cap;
+    const uint32_t snodes = uniform(P.heap_snodes ? P.heap_snodes : kHeapSmemNodes) - 1;  // per warp: buffer + nodes
+    hp.sn = snodes - 1;
+    hp.snodes = snodes_all + warp * snodes * 32;
+    hp.cap = uniform(d.heap_cap);
     // Bucket front: pages, links and free stacks in the instance's bucket
     // area; the push scratch (64 words per warp) in shared memory after the
     // heap nodes.
     Buckets<KW> bq;
-    {
-        const uint32_t BP = P.buckets ? d.bq_pages : 0u;
-        E* const pages_all = reinterpret_cast<E*>(d.bq_base);
-        uint32_t* const link_all = reinterpret_cast<uint32_t*>(pages_all + (size_t)H * BP * 32);
-        bq.P = BP;
-        bq.pages = pages_all + (size_t)hid * BP * 32;
-        bq.link = link_all + (size_t)hid * BP;
-        bq.fstack = link_all + (size_t)H * BP + (size_t)hid * BP;
-        bq.state = link_all + 2 * (size_t)H * BP + (size_t)hid * kBucketStateWords;
-        bq.upd = reinterpret_cast<uint32_t*>(snodes_all + (size_t)W * (hp.sn - 1) * 32) + (size_t)warp * 64;
-        bq_init(bq, lane);
-    }
+    bq.P = uniform(P.buckets ? d.bq_pages : 0u);
+    bq.pages = reinterpret_cast<E*>(d.bq_base) + (size_t)hid * bq.P * 32;
+    bq.upd = reinterpret_cast<uint32_t*>(snodes_all + W * snodes * 32) + warp * 64;
+    // Word tables of the bucket area, past every warp's pages: links, free
+    // stacks (as many words each), saved states.
+    auto bq_words = [&]() {
+        return reinterpret_cast<uint32_t*>(reinterpret_cast<E*>(d.bq_base) + (size_t)d.heaps * bq.P * 32);
+    };
+    bq.link = bq_words() + (size_t)hid * bq.P;
+    bq.fs_off = d.heaps * bq.P;
+    bq_init(bq, lane);
 
-    const uint32_t life = ld_vol(&ctl->life);
-    if (!multi && threadIdx.x < kSlots) {
-        TeamSlot& t = sm.slot[threadIdx.x];
-        t.minprio = kInfPrio;
-        t.minstage = kInfPrio;
-        t.count = 0;
-        t.best = kInf;
-        t.err = 0;
-    }
+    const uint32_t life = uniform(ld_vol(&ctl->life));
+    if (!multi && threadIdx.x < kSlots) slot_clear(sm.slot[threadIdx.x]);
+    if (lane < 3) sm.wcnt[warp][lane] = 0;
     uint32_t status = kInf;  // kInf while running / suspended
     uint32_t best_r;         // best goal cost seen (identical in every thread)
     bool have_prev;          // the previous iteration's slot holds the heaps' min
@@ -564,7 +542,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
         // (a length above the list's capacity means they were not) and few,
         // otherwise the whole table.  Listed offsets are the previous solve's, in the
         // same buffer; its table may have been larger than this solve's.
-        const uint64_t stride = (uint64_t)tm.ctas * blockDim.x;
+        const uint64_t stride = (uint64_t)(multi ? tm.ctas : 1u) * blockDim.x;
         const uint64_t tid = (uint64_t)rank * blockDim.x + threadIdx.x;
         // Where either clear will do, scattered stores costing about a
         // 32-byte sector each against streaming ones, the list is used while
@@ -584,47 +562,47 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
             if ((d.table_words & 1) && tid == 0)  // odd cell count: last word
                 __stcg(d.table + d.table_words - 1, kEmpty);
         }
-        heap_init(hp);
+        heap_init(hp, lane);
         if (!tsync()) status = ST_BARRIER;
         if (hid == 0) {
             E s = inf_entry<KW>();
             s.prio = make_prio(D::start_f(ctx, d), 0, kRootMove);
             D::set_key(s, ctx.start);
-            if (lane == 0) hp.part = s;
+            if (lane == 0) st_part(hp, 0, s);
+            __syncwarp();
             hp.pc = 1;
         }
         if (leader) {
-            uint64_t old, slot = 0;
-            D::insert(tab, ctx.start, make_val(0, D::kRootCode), old, slot);
+            uint64_t old;
+            uint32_t slot = 0;
+            D::insert(D::make_tab(d), ctx.start, make_val(0, D::kRootCode), old, slot);
             if (d.touched) {
                 *d.touched_count = 1;
-                d.touched[0] = (uint32_t)slot;
+                d.touched[0] = slot;
             }
             atomicAdd(&ctl->table_used, 1ull);
             ctl->t_start = globaltimer_ns();
         }
-        best_r = D::is_goal(ctx, ctx.start) ? 0u : kInf;
+        best_r = uniform_if(D::is_goal(ctx, ctx.start)) ? 0u : kInf;
         have_prev = true;  // the start is the only open entry; every slot starts empty
     } else {
-        heap_restore(hp, lane);
-        bq_restore(bq, lane);
-        best_r = ld_vol(&ctl->best);
+        heap_restore(hp, d.heap_hdr + 2 * hid, lane);
+        bq_restore(bq, bq_words() + 2 * (size_t)d.heaps * bq.P + (size_t)hid * kBucketStateWords, lane);
+        best_r = uniform(ld_vol(&ctl->best));
         have_prev = false;
     }
     // Multi-block teams: each block stages into its own region of the ring
     // buffers and aggregates its counters and minima in shared memory; thread
     // 0 publishes them (ready word, cut slot).
-    const size_t region_cap = stage_entries_per_buffer(W, ew_cap, MAXN);
+    E* const stage0 = multi ? reinterpret_cast<E*>(tm.stage) : reinterpret_cast<E*>(g_dyn_smem);
     unsigned long long* const ready =
-        multi ? reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(tm.stage) +
-                                                      (size_t)kStageRing * stage_cap * sizeof(E))
-              : nullptr;
+        multi ? reinterpret_cast<unsigned long long*>(stage0 + (size_t)kStageRing * tm.ctas * region_cap) : nullptr;
     if (multi && threadIdx.x == 0) {
         for (uint32_t r = 0; r < kStageRing; ++r) ready[(size_t)r * tm.ctas + rank] = 0;
         if (rank == 0)
             for (uint32_t k = 0; k < kCuts; ++k) {
                 CutSlot& c = tm.ctl->cut[k];
-                c.minprio = kInfPrio;
+                c.minf = kInf;
                 c.claims = c.exps = 0;
                 c.best = kInf;
                 c.lossy = c.err = c.count = 0;
@@ -632,53 +610,49 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
     }
     if (status == kInf && !tsync()) status = ST_BARRIER;
 
-    const uint32_t ew = d.ew;
     // This warp's current claim-list chunk (none reserved yet).
     unsigned long long t_base = 0;
     uint32_t t_used = kTouchedChunk;
-    uint32_t fmin = D::start_f(ctx, d);  // min f over the open list at the last check
+    uint32_t fmin = uniform(D::start_f(ctx, d));  // min f over the open list at the last check
     uint32_t it = 0;
-    const uint32_t it0 = ld_vol(&ctl->iterations);
+    const uint32_t slice = uniform(sm.slice);
+    const uint32_t it0 = uniform(ld_vol(&ctl->iterations));
     if (threadIdx.x == 0) {
-        sm.agg.minstage = kInfPrio;
-        sm.agg.best = kInf;
-        sm.agg.err = 0;
-        sm.agg.count = 0;
-        sm.agg_minprio = kInfPrio;
+        slot_clear(sm.agg);
+        sm.agg_minheap = kInf;
         sm.agg_err_prev = 0;
-        for (int i = 0; i < 5; ++i) sm.cnt[i] = 0;
         // Budgets are tested against these (no global reads per iteration).
         sm.base[0] = ld_vol64(&ctl->table_used);
         sm.base[1] = ld_vol64(&ctl->expansions);
         sm.t_start = *(const volatile uint64_t*)&ctl->t_start;
-        sm.pub[0] = sm.pub[1] = sm.run[0] = sm.run[1] = 0;
+        sm.run[0] = sm.run[1] = sm.mine[0] = sm.mine[1] = 0;
     }
     __syncthreads();
     // The first cut of a multi-block team holds the heaps as they are now.
     if (multi) {
-        const uint64_t mp = open_min(hp, bq);
-        if (lane == 0 && mp != kInfPrio) atomicMin(&sm.agg_minprio, (unsigned long long)mp);
+        const uint32_t mf = open_minf(hp, bq);
+        if (lane == 0 && mf != kInf) atomicMin(&sm.agg_minheap, mf);
     }
     while (status == kInf) {
-        const uint32_t s = it % kSlots;
-        TeamSlot* S = slots + s;
+        TeamSlot* const S = &sm.slot[it % kSlots];
         // Where this block's warps record the iteration: the team slot itself
         // for one-block teams (shared memory), the block aggregate otherwise.
-        TeamSlot* Sw = multi ? &sm.agg : S;
+        TeamSlot* const Sw = multi ? &sm.agg : S;
         E* const stage = multi ? stage0 + ((size_t)(it % kStageRing) * tm.ctas + rank) * region_cap
-                               : stage0 + (size_t)(it & 1) * stage_cap;
+                               : reinterpret_cast<E*>(g_dyn_smem) + (it & 1) * region_cap;
+        const typename D::Tab tab = D::make_tab(d);
         if (!multi && leader) {
             // One-block team: slot it+1 was last read right after the block
             // barrier of iteration it-2; every warp is past that point, and
             // none writes it before the barrier of this iteration.
-            TeamSlot* nx = slots + (it + 1) % kSlots;
-            nx->minprio = kInfPrio;
-            nx->minstage = kInfPrio;
-            nx->count = 0;
-            nx->best = kInf;
-            nx->err = 0;
-            if (sm.base[0] + sm.cnt[4] > d.table_limit) atomicCAS(&S->err, 0u, (uint32_t)ST_TABLE_FULL);
-            if (d.max_exp && sm.base[1] + sm.cnt[0] >= d.max_exp) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
+            slot_clear(sm.slot[(it + 1) % kSlots]);
+            if (it) {  // the previous iteration's counts are complete
+                const TeamSlot& pv = sm.slot[(it + kSlots - 1) % kSlots];
+                sm.run[0] += pv.claims;
+                sm.run[1] += pv.exps;
+            }
+            if (sm.base[0] + sm.run[0] > d.table_limit) atomicCAS(&S->err, 0u, (uint32_t)ST_TABLE_FULL);
+            if (d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
             if (d.max_iter && it0 + it + 1 >= d.max_iter) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
             if (d.timeout_ns && globaltimer_ns() - sm.t_start > d.timeout_ns)
                 atomicCAS(&S->err, 0u, (uint32_t)ST_TIMEOUT);
@@ -692,176 +666,226 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                                  : kInfPrio;
         E e;
         const uint32_t cnt =
-            open_pop(hp, bq, d.wide_after && it0 + it >= d.wide_after ? d.ew_wide : ew, lim, e, lane);
+            open_pop(hp, bq, uniform(d.wide_after && it0 + it >= d.wide_after ? d.ew_wide : d.ew), lim, e, lane);
         bool act = (uint32_t)lane < cnt;
         const KeyT k = D::key_of(e);
-        const uint32_t g = prio_g(e.prio), h = prio_f(e.prio) - g;
-        uint32_t pm = prio_pm(e.prio), self = 0;
-        bool stale = false;
-        uint32_t goal_g = kInf;
+        const uint32_t g = prio_g(e.prio);
+        uint32_t self = 0, goal_g = kInf, n_stale = 0;
         if (act && D::is_goal(ctx, k)) {
             // The goal is never expanded (a_star.h:80-83); its cost counts
             // unless a lower g for it is already known.
             if ((uint32_t)(D::get(tab, k) >> 32) >= g) goal_g = g;
             act = false;
         }
-        typename D::Look look{};
         if constexpr (D::kParentBySlot) {
             // Plugins record parents by slot: the entry's own slot is needed
             // before its successors are inserted.
-            if (act) {
-                const uint64_t v = D::get_self(tab, k, self);
-                pm = (uint32_t)v;
-                if ((uint32_t)(v >> 32) < g) {
-                    stale = true;
-                    act = false;
-                }
+            bool stale = false;
+            if (act && (uint32_t)(D::get_self(tab, k, self) >> 32) < g) {
+                stale = true;
+                act = false;
             }
-        } else {
-            if (act) look = D::look_begin(tab, k);  // resolved after the probes are in flight
+            n_stale = __popc(__ballot_sync(kFull, stale));
         }
 
-        // ---- expand: per group of moves, all successors, then all probes,
-        // then all atomicMins, so each group costs ~2 memory round trips ----
-        const typename D::Pre pre = D::prepare(ctx, k);
-        constexpr int GS = MAXN < 4 ? MAXN : 4;
-        uint32_t n_gen = 0, n_claim = 0, pushed = 0;
-        uint64_t smin = kInfPrio;
+        // ---- expand: one lane per (entry, move) ----
+        // Lane l of round r takes move l % LPE of entry r * EPR + l / LPE.
+        // Bound by round trips to L2/HBM and by the SM's rate of scattered
+        // accesses (measured per SM: one L2 load per cycle, one L2 atomic per
+        // 2.1, six cycles per random HBM sector); per round one probe
+        // instruction covers EPR whole neighbourhoods (a grid cell's three
+        // rows share sectors), RB rounds' probes are in flight together, and
+        // a warp that popped few entries runs few rounds.  A plain 4096^2
+        // grid pops four entries per warp and iteration: with one lane per
+        // entry and the moves in sequence its expansion took 8.9 k cycles of
+        // a 27 k cycle iteration, now 3.1 k of 18 k (74.4 -> 48.9 ms).  The
+        // lane of the move straight back to the parent, which has no
+        // successor, checks whether the entry is stale.
+        const uint32_t live = __ballot_sync(kFull, act);
+        // The popped lanes as a vote: the round tests below are then uniform
+        // branches to the compiler too.
+        const uint32_t popped = __ballot_sync(kFull, (uint32_t)lane < cnt);
+        const uint32_t lt = (1u << lane) - 1u;
+        const int sub = lane & (LPE - 1);
+        uint32_t n_gen = 0, n_claim = 0, pushed = 0, fstage = kInf;
         bool tfull = false, range = false;
+        for (uint32_t r0 = 0; r0 < (uint32_t)LPE && (popped >> (r0 * EPR)) != 0; r0 += RB) {
+#pragma unroll 1
+            for (int mg = 0; mg < MAXN; mg += LPE) {
+                const int m = mg + sub;
+                KeyT nk[RB];
+                uint32_t ng[RB], nf[RB], wt[RB];
+                uint64_t old[RB], seen[RB], own_v[RB];
+                uint32_t slot[RB];
+                uint32_t code[RB];  // parent as recorded in the table
+                bool ok[RB], own[RB];
+                // Issue: nothing here waits for a probe, so RB rounds' probes
+                // are in flight together.
 #pragma unroll
-        for (int g0 = 0; g0 < MAXN; g0 += GS) {
-            KeyT nk[GS];
-            uint32_t ng[GS], nh[GS];
-            bool ok[GS];
-#pragma unroll
-            for (int j = 0; j < GS; ++j) {
-                ok[j] = act && D::succ(ctx, k, pre, g0 + j, pm, g, h, nk[j], ng[j], nh[j]);
-                n_gen += ok[j];
-                if (ok[j] && ng[j] > kMaxG) {
-                    range = true;
-                    ok[j] = false;
-                }
-                ok[j] = ok[j] && ng[j] + nh[j] < best_r;  // cannot beat the best goal found
-            }
-            uint64_t slot[GS], old[GS], val[GS];
-            int cl[GS];
-#pragma unroll
-            for (int j = 0; j < GS; ++j) {
-                val[j] = make_val(ng[j], D::code(g0 + j, self));
-                old[j] = 0;
-                cl[j] = ok[j] ? D::claim_first(tab, nk[j], val[j], slot[j], old[j]) : -1;
-            }
-#pragma unroll
-            for (int j = 0; j < GS; ++j) {
-                if (cl[j] == 2) cl[j] = D::claim_probe(tab, nk[j], val[j], slot[j], old[j]);
-                if (ok[j] && cl[j] < 0) tfull = true;
-            }
-#pragma unroll
-            for (int j = 0; j < GS; ++j) {
-                if (cl[j] >= kClNeedMin) {
-                    old[j] = D::min_at(tab, slot[j], nk[j], val[j], old[j]);
-                    cl[j] -= kClNeedMin;
-                }
-            }
-            if constexpr (!D::kParentBySlot) {
-                if (g0 == 0 && act && (uint32_t)(D::look_end(tab, k, look) >> 32) < g) {
-                    // Stale: the table g went below the entry's own.  The
-                    // successors just inserted are real paths and stay in the
-                    // table but are not queued; the entry with the lower g
-                    // covers them.
-                    stale = true;
-                    act = false;
-                }
-            }
-            uint32_t nacc = 0, ncl = 0;
-            bool acc[GS], clm[GS];
-#pragma unroll
-            for (int j = 0; j < GS; ++j) {
-                const bool in = ok[j] && cl[j] >= 0;
-                acc[j] = in && act && (uint32_t)(old[j] >> 32) > ng[j];
-                clm[j] = in && cl[j] == 1;
-                nacc += acc[j];
-                ncl += clm[j];
-                if (acc[j]) {
-                    const uint64_t pr = make_prio(ng[j] + nh[j], ng[j], (uint32_t)(g0 + j));
-                    smin = pr < smin ? pr : smin;
-                    if (D::is_goal(ctx, nk[j]) && ng[j] < goal_g) goal_g = ng[j];
-                }
-            }
-            n_claim += ncl;
-            // Stage the improved successors: one atomic per warp reserves the range.
-            const uint32_t incl = warp_incl_sum(nacc, lane);
-            const uint32_t total = __shfl_sync(kFull, incl, 31);
-            if (total) {
-                uint32_t base = 0;
-                if (lane == 31) base = atomicAdd(&Sw->count, total);
-                base = __shfl_sync(kFull, base, 31) + incl - nacc;
-#pragma unroll
-                for (int j = 0; j < GS; ++j) {
-                    if (acc[j]) {
-                        E out = inf_entry<KW>();
-                        out.prio = make_prio(ng[j] + nh[j], ng[j], (uint32_t)(g0 + j));
-                        D::set_key(out, nk[j]);
-                        st_stage(stage + base++, out, multi);
+                for (int j = 0; j < RB; ++j) {
+                    ok[j] = own[j] = false;
+                    if (r0 + j >= (uint32_t)LPE || (popped >> ((r0 + j) * EPR)) == 0) continue;  // warp-uniform
+                    const int src = (int)((r0 + j) * EPR) + lane / LPE;
+                    const E x = shfl_idx(e, src);
+                    const KeyT xk = D::key_of(x);
+                    const uint32_t xg = prio_g(x.prio), pm = prio_pm(x.prio);
+                    uint32_t xself = 0, nh = 0;
+                    if constexpr (D::kParentBySlot) xself = __shfl_sync(kFull, self, src);
+                    const bool on = ((live >> src) & 1u) && m < MAXN;
+                    if constexpr (!D::kParentBySlot) own[j] = on && D::is_back(m, pm);
+                    ng[j] = xg;
+                    if constexpr (D::kDense) {
+                        // The neighbour's weight and value load together; a
+                        // value that is already as good needs no atomic
+                        // (four of five do not: 7.5 M of 9.8 M generated on
+                        // a 1021^2 grid), and a load costs half an atomic.
+                        ok[j] = on && !own[j] && D::step(ctx, xk, m, nk[j], nh);
+                        if (own[j]) nk[j] = xk;
+                        if (ok[j] || own[j]) old[j] = D::get(tab, nk[j]);
+                        if (ok[j]) wt[j] = D::weight(ctx, nk[j]);
+                        nf[j] = nh;
+                    } else {
+                        ok[j] = on && !own[j] && D::succ(ctx, xk, m, xg, prio_f(x.prio) - xg, nk[j], ng[j], nh);
+                        n_gen += __popc(__ballot_sync(kFull, ok[j]));
+                        if (ok[j] && ng[j] > kMaxG) {
+                            range = true;
+                            ok[j] = false;
+                        }
+                        nf[j] = ng[j] + nh;
+                        ok[j] = ok[j] && nf[j] < best_r;  // cannot beat the best goal found
+                        code[j] = D::code(m, xself);
+                        if (ok[j]) D::claim_begin(tab, nk[j], make_val(ng[j], code[j]), slot[j], seen[j], old[j]);
+                        if constexpr (!D::kParentBySlot) {
+                            if (own[j]) {
+                                nk[j] = xk;
+                                D::look_begin(tab, xk, seen[j], old[j], own_v[j]);
+                            }
+                        }
                     }
                 }
+                if constexpr (D::kDense) {
+#pragma unroll
+                    for (int j = 0; j < RB; ++j) {
+                        if (r0 + j >= (uint32_t)LPE || (popped >> ((r0 + j) * EPR)) == 0) continue;
+                        // Stale: the table's g went below the entry's own.
+                        const uint32_t sb = __ballot_sync(kFull, own[j] && (uint32_t)(old[j] >> 32) < ng[j]);
+                        const bool stale = (sb >> (lane & ~(LPE - 1)) & group_mask<LPE>()) != 0;
+                        n_stale += __popc(sb);
+                        ok[j] = ok[j] && !stale && wt[j] != 0;  // 0: obstacle
+                        n_gen += __popc(__ballot_sync(kFull, ok[j]));
+                        if (ok[j]) ng[j] += wt[j];
+                        if (ok[j] && ng[j] > kMaxG) {
+                            range = true;
+                            ok[j] = false;
+                        }
+                        nf[j] += ng[j];
+                        const uint64_t v = make_val(ng[j], (uint32_t)m);
+                        ok[j] = ok[j] && nf[j] < best_r && v < old[j];
+                        if (ok[j]) old[j] = D::lower(tab, nk[j], v);
+                    }
+                }
+                uint32_t acc_at[RB], clm_at[RB];
+                uint32_t total = 0, claimed = 0;
+#pragma unroll
+                for (int j = 0; j < RB; ++j) {
+                    acc_at[j] = clm_at[j] = kInf;
+                    if (r0 + j >= (uint32_t)LPE || (popped >> ((r0 + j) * EPR)) == 0) continue;
+                    bool stale = false;
+                    int cl = -1;
+                    if constexpr (D::kDense) {
+                        if (ok[j]) cl = old[j] == kEmpty ? 1 : 0;
+                    } else {
+                        if (ok[j]) cl = D::claim_end(tab, nk[j], make_val(ng[j], code[j]), slot[j], seen[j],
+                                                     old[j]);
+                        if (ok[j] && cl < 0) tfull = true;
+                        if constexpr (!D::kParentBySlot) {
+                            // A stale entry's successors are real paths and
+                            // stay in the table, but are not queued; the
+                            // entry with the lower g covers them.
+                            const bool st =
+                                own[j] && (uint32_t)(D::look_end(tab, nk[j], seen[j], old[j], own_v[j]) >> 32) < ng[j];
+                            const uint32_t sb = __ballot_sync(kFull, st);
+                            stale = (sb >> (lane & ~(LPE - 1)) & group_mask<LPE>()) != 0;
+                            n_stale += __popc(sb);
+                        }
+                    }
+                    const bool in = ok[j] && cl >= 0;
+                    const bool acc = in && !stale && (uint32_t)(old[j] >> 32) > ng[j];
+                    const uint32_t ab = __ballot_sync(kFull, acc), cb = __ballot_sync(kFull, in && cl == 1);
+                    if (acc) {
+                        acc_at[j] = total + __popc(ab & lt);
+                        fstage = nf[j] < fstage ? nf[j] : fstage;
+                        if (D::is_goal(ctx, nk[j]) && ng[j] < goal_g) goal_g = ng[j];
+                    }
+                    if (in && cl == 1) clm_at[j] = claimed + __popc(cb & lt);
+                    total += __popc(ab);
+                    claimed += __popc(cb);
+                }
+                n_claim += claimed;
                 pushed += total;
-            }
-            if (d.touched) {  // record claimed slots for the next solve's clear
-                const uint32_t ci = warp_incl_sum(ncl, lane);
-                const uint32_t ct = __shfl_sync(kFull, ci, 31);
-                if (ct) {
+                // Stage the improved successors: one atomic per warp reserves the range.
+                if (total) {
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(&Sw->count, total);
+                    base = __shfl_sync(kFull, base, 0);
+#pragma unroll
+                    for (int j = 0; j < RB; ++j) {
+                        if (acc_at[j] != kInf) {
+                            E out = inf_entry<KW>();
+                            out.prio = make_prio(nf[j], ng[j], (uint32_t)m);
+                            D::set_key(out, nk[j]);
+                            st_stage<multi>(stage + base + acc_at[j], out);
+                        }
+                    }
+                }
+                if (d.touched && claimed) {  // record claimed slots for the next solve's clear
                     // Fill the warp's chunk; a group that overruns it
                     // continues in a newly reserved one.
                     const uint32_t room = kTouchedChunk - t_used;
                     unsigned long long nb = 0;
-                    if (ct > room) {
+                    if (claimed > room) {
                         if (lane == 0) nb = atomicAdd(d.touched_count, (unsigned long long)kTouchedChunk);
                         nb = __shfl_sync(kFull, nb, 0);
                     }
-                    uint32_t pos = ci - ncl;
 #pragma unroll
-                    for (int j = 0; j < GS; ++j) {
-                        if (clm[j]) {
+                    for (int j = 0; j < RB; ++j) {
+                        if (clm_at[j] != kInf) {
+                            const uint32_t pos = clm_at[j];
                             const unsigned long long at = pos < room ? t_base + t_used + pos : nb + (pos - room);
-                            if (at < d.touched_cap) d.touched[at] = (uint32_t)slot[j];
-                            ++pos;
+                            if (at < d.touched_cap) d.touched[at] = slot[j];
                         }
                     }
-                    if (ct > room) {
+                    if (claimed > room) {
                         t_base = nb;
-                        t_used = ct - room;
+                        t_used = claimed - room;
                     } else {
-                        t_used += ct;
+                        t_used += claimed;
                     }
                 }
             }
         }
-        const unsigned bexp = __ballot_sync(kFull, act), bstale = __ballot_sync(kFull, stale);
+        __syncwarp();
         {
-            uint32_t gsum = n_gen, csum = n_claim;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                gsum += __shfl_xor_sync(kFull, gsum, o);
-                csum += __shfl_xor_sync(kFull, csum, o);
-                const uint32_t gg = __shfl_xor_sync(kFull, goal_g, o);
-                goal_g = gg < goal_g ? gg : goal_g;
-            }
-            smin = warp_min64(smin);
+            // The counts are warp-uniform; minima over the lanes with one
+            // reduction each.
+            const uint32_t smin = __reduce_min_sync(kFull, fstage);
+            goal_g = __reduce_min_sync(kFull, goal_g);
             const bool any_full = __any_sync(kFull, tfull), any_range = __any_sync(kFull, range);
             if (lane == 0) {
-                if (bexp) atomicAdd(&sm.cnt[0], (unsigned long long)__popc(bexp));
-                if (bstale) atomicAdd(&sm.cnt[1], (unsigned long long)__popc(bstale));
-                if (gsum) atomicAdd(&sm.cnt[2], (unsigned long long)gsum);
-                if (pushed) atomicAdd(&sm.cnt[3], (unsigned long long)pushed);
-                if (csum) atomicAdd(&sm.cnt[4], (unsigned long long)csum);
-                if (smin != kInfPrio) atomicMin(&Sw->minstage, (unsigned long long)smin);
+                const uint32_t n_exp = __popc(live) - (D::kParentBySlot ? 0u : n_stale);
+                sm.wcnt[warp][0] += n_stale;
+                sm.wcnt[warp][1] += n_gen;
+                sm.wcnt[warp][2] += pushed;
+                if (n_exp) atomicAdd(&Sw->exps, n_exp);
+                if (n_claim) atomicAdd(&Sw->claims, n_claim);
+                if (smin != kInf) atomicMin(&Sw->minstage, smin);
                 if (goal_g != kInf) atomicMin(&Sw->best, goal_g);
                 if (any_full) atomicCAS(&Sw->err, 0u, (uint32_t)ST_TABLE_FULL);
                 if (any_range) atomicCAS(&Sw->err, 0u, (uint32_t)ST_COST_RANGE);
             }
+            __syncwarp();
         }
-        if (multi) {
+        if constexpr (multi) {
             // ---- one hand-off per iteration: publish cut `it` and this
             // block's stage region, then wait for the region this block
             // pushes and test cut it - kCutLag (a_star.h:260-262) ----
@@ -881,7 +905,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                 if (leader) {
                     if (it >= 2 * kCutLag + 2) {  // every block has read it; none writes it yet
                         CutSlot* r = cuts + (it - 2 * kCutLag - 2) % kCuts;
-                        r->minprio = kInfPrio;
+                        r->minf = kInf;
                         r->claims = r->exps = 0;
                         r->best = kInf;
                         r->lossy = r->err = r->count = 0;
@@ -893,13 +917,12 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                 // (a superset of what is left after this iteration's pops) and
                 // what this iteration staged.
                 CutSlot* c = cuts + it % kCuts;
-                const unsigned long long cm =
-                    sm.agg_minprio < sm.agg.minstage ? sm.agg_minprio : sm.agg.minstage;
-                if (cm != kInfPrio) atomicMin(&c->minprio, cm);
-                if (sm.cnt[4] != sm.pub[0]) atomicAdd(&c->claims, sm.cnt[4] - sm.pub[0]);
-                if (sm.cnt[0] != sm.pub[1]) atomicAdd(&c->exps, sm.cnt[0] - sm.pub[1]);
-                sm.pub[0] = sm.cnt[4];
-                sm.pub[1] = sm.cnt[0];
+                const uint32_t cm = sm.agg_minheap < sm.agg.minstage ? sm.agg_minheap : sm.agg.minstage;
+                if (cm != kInf) atomicMin(&c->minf, cm);
+                if (sm.agg.claims) atomicAdd(&c->claims, (unsigned long long)sm.agg.claims);
+                if (sm.agg.exps) atomicAdd(&c->exps, (unsigned long long)sm.agg.exps);
+                sm.mine[0] += sm.agg.claims;
+                sm.mine[1] += sm.agg.exps;
                 if (sm.agg.best != kInf) atomicMin(&c->best, sm.agg.best);
                 if (lossy) atomicCAS(&c->lossy, 0u, lossy);
                 if (err) atomicCAS(&c->err, 0u, err);
@@ -912,11 +935,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                 fence_acq_rel_gpu();
                 st_relaxed_u64(rw + rank, ((unsigned long long)(it + 1) << 32) | mine);
                 red_relaxed_add_u32(&c->count, 1u);
-                sm.agg.best = kInf;
-                sm.agg.err = 0;
-                sm.agg.count = 0;
-                sm.agg.minstage = kInfPrio;
-                sm.agg_minprio = kInfPrio;
+                slot_clear(sm.agg);
+                sm.agg_minheap = kInf;
                 sm.agg_err_prev = 0;
                 uint32_t dec = kInf, n = 0, dbest = kInf, dfmin = kInf;
                 if (from == rank)
@@ -930,7 +950,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                     if (!team_wait_u32(&t->count, tm.ctas, tseen, tm.ctl, P.barrier_timeout_ns)) {
                         dec = ST_BARRIER;
                     } else {
-                        const uint64_t open_min = ld_vol64(&t->minprio);
+                        const uint32_t open_f = ld_vol(&t->minf);
                         dbest = ld_vol(&t->best);
                         uint32_t tl = ld_vol(&t->lossy), te = ld_vol(&t->err);
                         // Budgets from the team's totals, the same in every block.
@@ -940,10 +960,10 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                         if (!te && d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) te = ST_BUDGET;
                         const uint32_t bb = dbest < best_r ? dbest : best_r;
                         if (tl) dec = tl;  // an iteration that lost entries proves nothing
-                        else if (bb != kInf && bb <= prio_f(open_min)) dec = ST_OK;
+                        else if (bb != kInf && bb <= open_f) dec = ST_OK;
                         else if (te) dec = te;
-                        else if (open_min == kInfPrio) dec = ST_NO_PATH;
-                        if (open_min != kInfPrio) dfmin = prio_f(open_min);
+                        else if (open_f == kInf) dec = ST_NO_PATH;
+                        dfmin = open_f;
                     }
                 }
                 sm.dec_status = dec;
@@ -953,10 +973,10 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
             }
             __syncthreads();
             {
-                const uint32_t db = sm.dec_best;
+                const uint32_t db = uniform(sm.dec_best), df = uniform(sm.dec_fmin);
                 best_r = db < best_r ? db : best_r;
-                if (sm.dec_fmin != kInf) fmin = sm.dec_fmin;
-                status = sm.dec_status;
+                if (df != kInf) fmin = df;
+                status = uniform(sm.dec_status);
             }
             if (status != kInf) break;
         } else {
@@ -967,23 +987,23 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
             // ---- termination test (a_star.h:260-262), one iteration behind ----
             // Open entries now: heaps after the previous push (>= that slot's
             // min) minus this iteration's pops, plus this iteration's stage.
-            const uint32_t sb = ld_vol(&S->best);
+            const uint32_t sb = uniform(ld_vol(&S->best));
             best_r = sb < best_r ? sb : best_r;
-            uint32_t err = ld_vol(&S->err);
-            uint64_t open_min = ld_vol64(&S->minstage);
+            uint32_t err = uniform(ld_vol(&S->err));
+            uint32_t open_f = uniform(ld_vol(&S->minstage));
             if (have_prev) {
-                const TeamSlot* pv = slots + (it + kSlots - 1) % kSlots;
-                if (!err) err = ld_vol(&pv->err);
-                const uint64_t mp = ld_vol64(&pv->minprio);
-                open_min = mp < open_min ? mp : open_min;
+                const TeamSlot* pv = &sm.slot[(it + kSlots - 1) % kSlots];
+                const uint32_t pe = uniform(ld_vol(&pv->perr)), mf = uniform(ld_vol(&pv->minheap));
+                if (!err) err = pe;
+                open_f = mf < open_f ? mf : open_f;
             }
             // An iteration that lost entries (full table or heap) proves nothing.
             if (err == ST_TABLE_FULL || err == ST_HEAP_FULL || err == ST_COST_RANGE) status = err;
-            else if (have_prev && best_r != kInf && best_r <= prio_f(open_min)) status = ST_OK;
+            else if (have_prev && best_r != kInf && best_r <= open_f) status = ST_OK;
             else if (err) status = err;
-            else if (have_prev && open_min == kInfPrio) status = ST_NO_PATH;
+            else if (have_prev && open_f == kInf) status = ST_NO_PATH;
             if (status != kInf) break;
-            if (open_min != kInfPrio) fmin = prio_f(open_min);
+            if (open_f != kInf) fmin = open_f;
         }
 
         // ---- push ----
@@ -995,43 +1015,42 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
             uint32_t total;
             const E* src;
             uint32_t first, step;
-            if (multi) {
+            if constexpr (multi) {
                 const uint32_t from = (rank + it) % tm.ctas;
-                total = sm.push_count;
+                total = uniform(sm.push_count);
                 src = stage0 + ((size_t)(it % kStageRing) * tm.ctas + from) * region_cap;
                 first = ((uint32_t)warp + it) % (uint32_t)W;
                 step = (uint32_t)W;
             } else {
-                total = ld_vol(&S->count);
+                total = uniform(ld_vol(&S->count));
                 src = stage;
-                first = (hid + H - it % H) % H;
-                step = H;
+                first = ((uint32_t)warp + (uint32_t)W - it % (uint32_t)W) % (uint32_t)W;
+                step = (uint32_t)W;
             }
-            const uint32_t nch = (total + 31) / 32;
+            // Chunks of up to 32 entries, smaller when that gives every warp
+            // of the block a share: a warp expands its pops in rounds.
+            const uint32_t per = (total + (uint32_t)W - 1) / (uint32_t)W;
+            const uint32_t cs = per < 32 ? per : 32u;
+            const uint32_t nch = cs ? (total + cs - 1) / cs : 0u;
             bool hfull = false;
             for (uint32_t c = first; c < nch; c += step) {
-                const uint32_t idx = c * 32 + (uint32_t)lane;
-                E x = idx < total ? ld_stage(src + idx, multi) : inf_entry<KW>();
-                const uint32_t m = total - c * 32 < 32 ? total - c * 32 : 32;
+                const uint32_t idx = c * cs + (uint32_t)lane;
+                const uint32_t m = total - c * cs < cs ? total - c * cs : cs;
+                E x = (uint32_t)lane < m ? ld_stage<multi>(src + idx) : inf_entry<KW>();
                 if (!open_push(hp, bq, x, m, lane)) {
                     hfull = true;
                     break;
                 }
             }
-            const uint64_t mp = open_min(hp, bq);
+            const uint32_t mf = open_minf(hp, bq);
             if (lane == 0) {
-                if (multi) {
-                    atomicMin(&sm.agg_minprio, (unsigned long long)mp);
-                    if (hfull) atomicCAS(&sm.agg_err_prev, 0u, (uint32_t)ST_HEAP_FULL);
-                } else {
-                    atomicMin(&S->minprio, (unsigned long long)mp);
-                    if (hfull) atomicCAS(&S->err, 0u, (uint32_t)ST_HEAP_FULL);
-                }
+                atomicMin(multi ? &sm.agg_minheap : &S->minheap, mf);
+                if (hfull) atomicCAS(multi ? &sm.agg_err_prev : &S->perr, 0u, (uint32_t)ST_HEAP_FULL);
             }
         }
         ++it;
         have_prev = true;
-        if (sm.slice && it >= sm.slice) break;  // suspend
+        if (slice && it >= slice) break;  // suspend
     }
 
     if (lane == 0) atomicMax(&ctl->max_nodes, hp.max_n);
@@ -1041,19 +1060,28 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
     {  // this launch's counters
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (sm.cnt[0]) atomicAdd(&ctl->expansions, sm.cnt[0]);
-            if (sm.cnt[1]) atomicAdd(&ctl->stale, sm.cnt[1]);
-            if (sm.cnt[2]) atomicAdd(&ctl->generated, sm.cnt[2]);
-            if (sm.cnt[3]) atomicAdd(&ctl->pushes, sm.cnt[3]);
-            if (sm.cnt[4]) atomicAdd(&ctl->table_used, sm.cnt[4]);
-            for (int i = 0; i < 5; ++i) sm.cnt[i] = 0;
+            if constexpr (!multi) {
+                // Iterations 0 .. it - 1 were counted when the next one began;
+                // the one the loop left by, or the last before a suspension:
+                const uint32_t last = status == kInf ? it - 1 : it;
+                const TeamSlot& t = sm.slot[last % kSlots];
+                sm.mine[0] = sm.run[0] + t.claims;
+                sm.mine[1] = sm.run[1] + t.exps;
+            }
+            if (sm.mine[1]) atomicAdd(&ctl->expansions, sm.mine[1]);
+            if (sm.mine[0]) atomicAdd(&ctl->table_used, sm.mine[0]);
+        }
+        if (lane == 0) {
+            if (sm.wcnt[warp][0]) atomicAdd(&ctl->stale, sm.wcnt[warp][0]);
+            if (sm.wcnt[warp][1]) atomicAdd(&ctl->generated, sm.wcnt[warp][1]);
+            if (sm.wcnt[warp][2]) atomicAdd(&ctl->pushes, sm.wcnt[warp][2]);
         }
     }
     if (status == kInf) {
         // Suspending: fold in what the iterations not tested yet found -- a
         // goal popped there is in no heap any more -- and stop on entries
         // they lost.
-        if (multi) {
+        if constexpr (multi) {
             if (threadIdx.x == 0) {
                 CutSlot* c = tm.ctl->cut + it % kCuts;
                 if (sm.agg.best != kInf) atomicMin(&c->best, sm.agg.best);
@@ -1075,25 +1103,23 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
                     sm.dec_status = lossy ? lossy : kInf;
                 }
                 __syncthreads();
-                best_r = sm.dec_best;
-                status = sm.dec_status;
+                best_r = uniform(sm.dec_best);
+                status = uniform(sm.dec_status);
             }
-        } else if (it > 0 && ld_vol(&slots[(it + kSlots - 1) % kSlots].err) == ST_HEAP_FULL) {
+        } else if (it > 0 && uniform(ld_vol(&sm.slot[(it + kSlots - 1) % kSlots].perr)) == ST_HEAP_FULL) {
             status = ST_HEAP_FULL;  // raised by the last push
         }
     }
     if (status == kInf) {  // suspended: keep the search state resident
-        heap_save(hp, lane);
-        bq_save(bq, lane);
+        heap_save(hp, d.heap_hdr + 2 * hid, lane);
+        bq_save(bq, bq_words() + 2 * (size_t)d.heaps * bq.P + (size_t)hid * kBucketStateWords, lane);
         if (leader) {
             ctl->best = best_r;
             ctl->iterations = it0 + it;
             __threadfence();
             ctl->life = LIFE_RUNNING;
         }
-        return;
-    }
-    if (leader) {
+    } else if (leader) {
         ctl->best = best_r;
         ctl->iterations = it0 + it;
         ctl->status = status;
@@ -1101,22 +1127,26 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const InstDesc&
         __threadfence();
         ctl->life = LIFE_DONE;
     }
+    // The callers' next block barrier wants whole warps: this function is not
+    // inlined, and a lane that returned ahead of the leader's would reach it
+    // alone.
+    __syncwarp();
 }
 
-template <uint32_t KINDS>
-__device__ __forceinline__ void dispatch(const LaunchParams& P, CtaShared& sm, const TeamRef tm) {
-    switch (sm.desc.kind) {
+template <uint32_t KINDS, int MAXT, int TEAM>
+__device__ __forceinline__ void dispatch(const LaunchParams& P, const TeamRef tm) {
+    switch (cta().desc.kind) {
         case KIND_SLIDING3:
-            if constexpr ((KINDS & kind_bit(KIND_SLIDING3)) != 0) run_instance<SlidingDom<3>>(P, sm.desc, sm, sm.ctx.s3, tm);
+            if constexpr ((KINDS & kind_bit(KIND_SLIDING3)) != 0) run_instance<SlidingDom<3>, MAXT, TEAM>(P, tm);
             break;
         case KIND_SLIDING4:
-            if constexpr ((KINDS & kind_bit(KIND_SLIDING4)) != 0) run_instance<SlidingDom<4>>(P, sm.desc, sm, sm.ctx.s4, tm);
+            if constexpr ((KINDS & kind_bit(KIND_SLIDING4)) != 0) run_instance<SlidingDom<4>, MAXT, TEAM>(P, tm);
             break;
         case KIND_SLIDING5:
-            if constexpr ((KINDS & kind_bit(KIND_SLIDING5)) != 0) run_instance<SlidingDom<5>>(P, sm.desc, sm, sm.ctx.s5, tm);
+            if constexpr ((KINDS & kind_bit(KIND_SLIDING5)) != 0) run_instance<SlidingDom<5>, MAXT, TEAM>(P, tm);
             break;
         case KIND_GRID:
-            if constexpr ((KINDS & kind_bit(KIND_GRID)) != 0) run_instance<GridDom>(P, sm.desc, sm, sm.ctx.g, tm);
+            if constexpr ((KINDS & kind_bit(KIND_GRID)) != 0) run_instance<GridDom, MAXT, TEAM>(P, tm);
             break;
         default:
             break;
@@ -1125,34 +1155,37 @@ __device__ __forceinline__ void dispatch(const LaunchParams& P, CtaShared& sm, c
 
 // Persistent search kernel.
 //  * plain (team_ctas > 1): every block works on instance 0 (cooperative launch);
-//  * batch/serve: blocks of the heavy teams first take heavy instances together,
-//    then every block takes instances one block each from a work counter.
+//  * batch/serve: blocks of the heavy teams first take heavy instances together
+//    (grids), then every block takes instances one block each from a work counter.
 // MAXT bounds the block size: 256 threads (8 warps) leave the compiler up to
-// 255 registers per thread, no spills; the all-kinds kernel has a second
-// instantiation for 16-warp blocks (batch/serve), capped at 128 registers.
+// 255 registers per thread; the all-kinds kernel has a second instantiation
+// for 16-warp blocks (batch/serve), capped at 128 registers.
 template <uint32_t KINDS, int MAXT = 256>
-__global__ void __launch_bounds__(MAXT, 1) search_kernel(LaunchParams P) {
-    __shared__ CtaShared sm;
-    if (P.team_ctas > 1) {
+__global__ void __launch_bounds__(MAXT, 1) search_kernel(const __grid_constant__ LaunchParams P) {
+    CtaShared& sm = cta();
+    // Single-kind kernels are the plain engine's; the all-kinds kernel of
+    // 16-warp blocks serves both.
+    constexpr bool plain = KINDS != kKindsAll || MAXT > 256, many = KINDS == kKindsAll;
+    if (plain && P.team_ctas > 1) {
         if (threadIdx.x == 0) {
             sm.desc = P.insts[0];
             sm.slice = P.slice_iters;
         }
         __syncthreads();
-        dispatch<KINDS>(P, sm, TeamRef{P.team_ctas, blockIdx.x, P.team, P.stage});
+        if constexpr (plain) dispatch<KINDS, MAXT, TEAM_RING>(P, TeamRef{P.team_ctas, blockIdx.x, P.team, P.stage});
         return;
     }
-    if (P.n_heavy && blockIdx.x < P.heavy_teams * P.heavy_team) {
+    if (many && P.n_heavy && blockIdx.x < P.heavy_teams * P.heavy_team) {
         const uint32_t t = blockIdx.x / P.heavy_team, rank = blockIdx.x % P.heavy_team;
         TeamCtl* tc = P.heavy_ctl + t;
         const TeamRef tm{P.heavy_team, rank, tc,
                          reinterpret_cast<char*>(P.heavy_stage) + (size_t)t * P.heavy_stage_bytes};
         for (;;) {
             // Every block of the team is done with the previous instance here.
-            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns, sm)) break;
+            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
             if (rank == 0 && threadIdx.x == 0) {
                 for (uint32_t k = 0; k < kCuts; ++k) {
-                    tc->cut[k].minprio = kInfPrio;
+                    tc->cut[k].minf = kInf;
                     tc->cut[k].claims = tc->cut[k].exps = 0;
                     tc->cut[k].best = kInf;
                     tc->cut[k].lossy = 0;
@@ -1161,7 +1194,7 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(LaunchParams P) {
                 }
                 tc->inst = atomicAdd(P.heavy_next, 1u);
             }
-            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns, sm)) break;
+            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
             const uint32_t i = ld_vol(&tc->inst);
             if (i >= P.n_heavy) break;
             if (threadIdx.x == 0) {
@@ -1170,12 +1203,14 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(LaunchParams P) {
                 sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
             }
             __syncthreads();
-            dispatch<KINDS>(P, sm, tm);
+            if constexpr (many) dispatch<kind_bit(KIND_GRID), MAXT, TEAM_RING>(P, tm);
+            __syncwarp();
         }
         __syncthreads();
     }
     for (;;) {
         if (threadIdx.x == 0) sm.inst = atomicAdd(P.next, 1u);
+        __syncwarp();
         __syncthreads();
         const uint32_t i = sm.inst;
         if (i >= P.n_insts) break;
@@ -1184,8 +1219,10 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(LaunchParams P) {
             sm.desc = P.insts[slot];
             sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
         }
+        __syncwarp();
         __syncthreads();
-        dispatch<KINDS>(P, sm, TeamRef{1, 0, nullptr, nullptr});
+        dispatch<KINDS, MAXT, TEAM_BLOCK>(P, TeamRef{1, 0, nullptr, nullptr});
+        __syncwarp();
         __syncthreads();
     }
 }
@@ -1275,9 +1312,6 @@ template <int N> __device__ void sliding_ctx_min(typename SlidingDom<N>::Ctx& c,
 // start, so the window is placed with the current cell kPathMargin cells from
 // its edge away from the start: up to ~28 steps per load.
 constexpr int kPathWin = 32, kPathMargin = 3, kPathWarps = 4;
-// GridDom::dx(m) + 1 and GridDom::dy(m) + 1 in bits 2m..2m+1.
-constexpr uint32_t kGridDxPack = 2u | 0u << 2 | 1u << 4 | 1u << 6 | 2u << 8 | 2u << 10 | 0u << 12 | 0u << 14;
-constexpr uint32_t kGridDyPack = 1u | 1u << 2 | 2u << 4 | 0u << 6 | 2u << 8 | 0u << 10 | 2u << 12 | 0u << 14;
 
 static __device__ __forceinline__ int path_win_origin(int c, int s, int n) {
     int o = s < c ? c - (kPathWin - 1 - kPathMargin) : s > c ? c - kPathMargin : c - kPathWin / 2;
