@@ -38,8 +38,9 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
     return x;
 }
 
-// Priority word: f in bits 63..32, (2^24-1 - g) in bits 31..8 and the move
-// that produced the entry in bits 7..0, so that one unsigned comparison gives
+// Priority word: f in bits 63..32, (2^24-1 - g) in bits 31..8 and a tag of
+// the domain in bits 7..0 (the move that produced the entry; puzzles: with the
+// blank's cell), so that one unsigned comparison gives
 // the reference's order "lower f first, equal f -> higher g first"
 // (QueueValue::operator<, a_star.h:58-63) and a popped entry knows its parent
 // move without a table lookup.  Costs are limited to kMaxG.
@@ -241,12 +242,25 @@ template <int KW> struct WarpHeap {
     uint32_t cap;       // tree nodes available (>= sn)
     uint32_t sn;        // nodes below sn live in shared memory
     uint32_t N;         // full nodes in the tree (warp-uniform)
-    uint32_t pc;        // entries in the partial buffer (warp-uniform), ascending; inf entries after
+    uint32_t pc;        // entries in the partial buffer (warp-uniform)
+    uint32_t pf;        // their least f (kInf: none; warp-uniform)
     uint32_t max_n;     // high-water mark of N
+    bool sorted;        // they are in ascending order (warp-uniform)
 };
 
+// The partial buffer collects pushes in arrival order and is sorted only when
+// a pop needs its best entries or it overflows into the tree: a search that
+// keeps a warp at a few entries per iteration (grids, small puzzles) then
+// neither sorts nor merges anything.
 template <int KW> __device__ __forceinline__ Entry<KW> ld_part(const WarpHeap<KW>& h, int lane) {
-    return ld_stage<false>(h.snodes + lane);
+    return (uint32_t)lane < h.pc ? ld_stage<false>(h.snodes + lane) : inf_entry<KW>();
+}
+template <int KW> __device__ __forceinline__ Entry<KW> ld_part_sorted(const WarpHeap<KW>& h, int lane) {
+    const Entry<KW> p = ld_part(h, lane);
+    return h.sorted ? p : sort32(p, lane);
+}
+template <int KW> __device__ __forceinline__ uint32_t least_f(const Entry<KW>& e) {
+    return __reduce_min_sync(kFull, prio_f(e.prio));
 }
 template <int KW> __device__ __forceinline__ void st_part(const WarpHeap<KW>& h, int lane, const Entry<KW>& e) {
     st_stage<false>(h.snodes + lane, e);
@@ -276,12 +290,12 @@ template <int KW> __device__ __forceinline__ void prefetch_node(const WarpHeap<K
     }
 }
 
-template <int KW> __device__ __forceinline__ void heap_init(WarpHeap<KW>& h, int lane) {
+template <int KW> __device__ __forceinline__ void heap_init(WarpHeap<KW>& h) {
     h.N = 0;
     h.pc = 0;
+    h.pf = kInf;
     h.max_n = 0;
-    st_part(h, lane, inf_entry<KW>());
-    __syncwarp();
+    h.sorted = true;
 }
 
 // `hdr`: the heap's saved {N, pc}.
@@ -289,7 +303,10 @@ template <int KW> __device__ __forceinline__ void heap_restore(WarpHeap<KW>& h, 
     h.N = uniform(__ldcg(hdr));
     h.pc = uniform(__ldcg(hdr + 1));
     h.max_n = h.N;
-    st_part(h, lane, (uint32_t)lane < h.pc ? ld_entry(h.nodes + (size_t)h.cap * 32 + lane) : inf_entry<KW>());
+    const Entry<KW> part = (uint32_t)lane < h.pc ? ld_entry(h.nodes + (size_t)h.cap * 32 + lane) : inf_entry<KW>();
+    st_part(h, lane, part);
+    h.pf = least_f(part);
+    h.sorted = false;
     for (uint32_t i = 0; i < h.N && i < h.sn; ++i) st_node(h, i, lane, ld_entry(h.nodes + (size_t)i * 32 + lane));
     __syncwarp();
 }
@@ -304,12 +321,11 @@ template <int KW> __device__ __forceinline__ void heap_save(const WarpHeap<KW>& 
     }
 }
 
-// Least priority of the heap (kInfPrio when it is empty; the warp calls it
-// after the last change is visible to every lane).
-template <int KW> __device__ __forceinline__ uint64_t heap_min(const WarpHeap<KW>& h) {
-    const uint64_t r = h.N ? *reinterpret_cast<const volatile uint64_t*>(&h.snodes[32].prio) : kInfPrio;
-    const uint64_t p = h.pc ? *reinterpret_cast<const volatile uint64_t*>(&h.snodes[0].prio) : kInfPrio;
-    return r < p ? r : p;
+// Least f of the heap (kInf when it is empty; the warp calls it after the
+// last change is visible to every lane).
+template <int KW> __device__ __forceinline__ uint32_t heap_minf(const WarpHeap<KW>& h) {
+    const uint32_t r = h.N ? prio_f(*reinterpret_cast<const volatile uint64_t*>(&h.snodes[32].prio)) : kInf;
+    return r < h.pf ? r : h.pf;
 }
 
 // Restores the node order from the root (new content `cur`, not stored yet) down.
@@ -359,17 +375,35 @@ template <int KW> __device__ void heap_sift_down(WarpHeap<KW>& h, Entry<KW> cur,
 // l < return value receives one.  Nothing changes when no entry qualifies.
 template <int KW>
 __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW>& out, int lane) {
-    const Entry<KW> part = ld_part(h, lane);
     if (h.N == 0) {
-        const uint32_t below = __popc(__ballot_sync(kFull, (uint32_t)lane < h.pc && part.prio < lim));
-        const uint32_t c = E < below ? E : below;
+        Entry<KW> part = ld_part(h, lane);
+        const uint32_t bm = __ballot_sync(kFull, part.prio < lim);
+        uint32_t c = __popc(bm);
+        if (c > E) {  // the E best of them
+            if (!h.sorted) part = sort32(part, lane);
+            h.sorted = true;
+            c = E;
+        } else if (c && c < h.pc && !h.sorted) {  // all of them, moved to the front
+            const uint32_t below = bm & ((1u << lane) - 1u);
+            const uint32_t to = (bm >> lane & 1u) ? __popc(below) : c + (uint32_t)lane - __popc(below);
+            __syncwarp();
+            if ((uint32_t)lane < h.pc) st_stage<false>(h.snodes + to, part);
+            __syncwarp();
+            part = ld_part(h, lane);
+        }
         out = (uint32_t)lane < c ? part : inf_entry<KW>();
-        Entry<KW> s = shfl_idx(part, (lane + (int)c) & 31);
-        st_part(h, lane, ((uint32_t)lane + c < h.pc) ? s : inf_entry<KW>());
-        h.pc -= c;
-        __syncwarp();
+        if (c) {
+            const Entry<KW> t = shfl_idx(part, (lane + (int)c) & 31);
+            const Entry<KW> rest = (uint32_t)lane + c < h.pc ? t : inf_entry<KW>();
+            h.pc -= c;
+            st_part(h, lane, rest);
+            h.pf = least_f(rest);
+            __syncwarp();
+        }
         return c;
     }
+    const Entry<KW> part = ld_part_sorted(h, lane);
+    h.sorted = true;  // every way on stores it back in order, but for the one that changes nothing
     prefetch_node(h, h.N - 1, lane);  // the last node refills the root when the buffer runs short
     Entry<KW> lo, hi;
     merge2(ld_node(h, 0, lane), part, lo, hi, lane);
@@ -377,6 +411,8 @@ __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW
         const uint32_t below = __popc(__ballot_sync(kFull, lo.prio < lim));
         if (below < E) E = below;
         if (E == 0) {
+            st_part(h, lane, part);
+            __syncwarp();
             out = inf_entry<KW>();
             return 0;
         }
@@ -391,11 +427,13 @@ __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW
     if (rest >= 32) {
         st_part(h, lane, r2);
         h.pc = rest - 32;
+        h.pf = least_f(r2);
         heap_sift_down(h, r1, lane);
     } else if (h.N == 1) {
         h.N = 0;
         st_part(h, lane, r1);
         h.pc = rest;
+        h.pf = least_f(r1);
         __syncwarp();
     } else {
         Entry<KW> last = ld_node(h, h.N - 1, lane);
@@ -404,6 +442,7 @@ __device__ uint32_t heap_pop(WarpHeap<KW>& h, uint32_t E, uint64_t lim, Entry<KW
         merge2(last, r1, lo2, hi2, lane);
         st_part(h, lane, hi2);
         h.pc = rest;
+        h.pf = least_f(hi2);
         heap_sift_down(h, lo2, lane);
     }
     return E;
@@ -441,26 +480,32 @@ template <int KW> __device__ bool heap_insert_node(WarpHeap<KW>& h, Entry<KW> F,
     return true;
 }
 
-// Pushes up to 32 entries (lanes >= m must hold padding entries).
+// Pushes the entries of the lanes in `mask` (the other lanes hold padding
+// entries).
 template <int KW>
-__device__ bool heap_push(WarpHeap<KW>& h, Entry<KW> x, uint32_t m, int lane) {
-    if (m == 0) return true;
-    x = sort32(x, lane);
-    Entry<KW> lo, hi;
-    merge2(ld_part(h, lane), x, lo, hi, lane);
-    const uint32_t tot = h.pc + m;
+__device__ bool heap_push(WarpHeap<KW>& h, Entry<KW> x, uint32_t mask, int lane) {
+    const uint32_t tot = h.pc + __popc(mask);
     if (tot < 32) {
-        st_part(h, lane, lo);
+        if (mask >> lane & 1u) st_stage<false>(h.snodes + h.pc + __popc(mask & ((1u << lane) - 1u)), x);
+        const uint32_t f = least_f(x);
+        h.pf = f < h.pf ? f : h.pf;
         h.pc = tot;
+        h.sorted = false;
         __syncwarp();
         return true;
     }
+    x = sort32(x, lane);
+    Entry<KW> lo, hi;
+    merge2(ld_part_sorted(h, lane), x, lo, hi, lane);
     // The largest 32 form a new node; the smallest stay in the partial buffer,
     // where the next pop sees them first.
     const uint32_t off = tot - 32;
     Entry<KW> node = pick(lo, hi, (int)off + lane);
-    st_part(h, lane, (uint32_t)lane < off ? lo : inf_entry<KW>());
+    const Entry<KW> rest = (uint32_t)lane < off ? lo : inf_entry<KW>();
+    st_part(h, lane, rest);
     h.pc = off;
+    h.pf = least_f(rest);
+    h.sorted = true;
     return heap_insert_node(h, node, lane);
 }
 
@@ -518,7 +563,7 @@ template <int KW> __device__ __forceinline__ uint32_t bq_min_f(const Buckets<KW>
 
 // Least f over a warp's open list (kInf when it is empty).
 template <int KW> __device__ __forceinline__ uint32_t open_minf(const WarpHeap<KW>& h, const Buckets<KW>& q) {
-    const uint32_t hf = prio_f(heap_min(h));
+    const uint32_t hf = heap_minf(h);
     if (!q.P) return hf;
     const uint32_t bf = bq_min_f(q);
     return hf < bf ? hf : bf;
@@ -615,7 +660,7 @@ __device__ bool open_push(WarpHeap<KW>& h, Buckets<KW>& q, Entry<KW> x, uint32_t
     const bool rest = valid && !placed;
     const uint32_t rm = __ballot_sync(kFull, rest);
     if (!rm) return true;
-    return heap_push(h, rest ? x : inf_entry<KW>(), (uint32_t)__popc(rm), lane);
+    return heap_push(h, rest ? x : inf_entry<KW>(), rm, lane);
 }
 
 // Pops up to E (1..32) entries with priority below `lim` (a multiple of 2^32
@@ -627,12 +672,12 @@ __device__ uint32_t open_pop(WarpHeap<KW>& h, Buckets<KW>& q, uint32_t E, uint64
     out = inf_entry<KW>();
     uint32_t taken = 0;
     for (int round = 0; round < 4 && taken < E; ++round) {
-        const uint32_t bf = bq_min_f(q);
-        const uint64_t hm = heap_min(h);
+        const uint32_t bf = bq_min_f(q), hf = uniform(heap_minf(h));
+        const uint32_t mf = hf < bf ? hf : bf;
+        if (mf == kInf || ((uint64_t)mf << 32) >= lim) break;
         const uint64_t bp = bf == kInf ? kInfPrio : ((uint64_t)bf << 32);
-        if (uniform_if((hm < bp ? hm : bp) >= lim)) break;
         const uint32_t i = (uint32_t)lane - taken;  // this lane's index among the new ones
-        if (uniform_if(hm < bp)) {  // the heap holds lower f: take its entries below the buckets' f
+        if (hf < bf) {  // the heap holds lower f: take its entries below the buckets' f
             Entry<KW> e;
             const uint32_t c = heap_pop(h, E - taken, bp < lim ? bp : lim, e, lane);
             const Entry<KW> sh = shfl_idx(e, (lane - (int)taken) & 31);

@@ -73,18 +73,14 @@ bool DevBuf::ensure(size_t bytes) {
     return true;
 }
 
-template <uint32_t K, int T = 256> const void* kernel_ptr() {
-    return reinterpret_cast<const void*>(&search_kernel<K, T>);
-}
-
 const void* search_kernel_for(uint32_t kinds, uint32_t threads) {
-    if (threads > 256) return kernel_ptr<kKindsAll, 512>();  // 9..16 warps: all kinds
+    if (threads > 256) return search_kernel_all16();  // 9..16 warps: all kinds
     switch (kinds) {
-        case kind_bit(KIND_SLIDING3): return kernel_ptr<kind_bit(KIND_SLIDING3)>();
-        case kind_bit(KIND_SLIDING4): return kernel_ptr<kind_bit(KIND_SLIDING4)>();
-        case kind_bit(KIND_SLIDING5): return kernel_ptr<kind_bit(KIND_SLIDING5)>();
-        case kind_bit(KIND_GRID): return kernel_ptr<kind_bit(KIND_GRID)>();
-        default: return kernel_ptr<kKindsAll>();
+        case kind_bit(KIND_SLIDING3): return search_kernel_sliding3();
+        case kind_bit(KIND_SLIDING4): return search_kernel_sliding4();
+        case kind_bit(KIND_SLIDING5): return search_kernel_sliding5();
+        case kind_bit(KIND_GRID): return search_kernel_grid();
+        default: return search_kernel_all();
     }
 }
 
@@ -137,6 +133,29 @@ int occupancy_blocks(gastar_ctx* /*c: the current device's context*/, uint32_t k
     return nb;
 }
 
+int occupancy_clusters(uint32_t kinds, uint32_t threads, size_t smem, uint32_t size) {
+    const void* f = search_kernel_for(kinds, threads);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(size);
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if ((smem > kSmemNoOptIn &&
+         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
+        (size > 8 && cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&n, f, &lc) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 int launch_search(gastar_ctx* /*c: the current device's context*/, uint32_t kinds, const LaunchParams& P,
                   uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t st) {
     const void* f = search_kernel_for(kinds, threads);
@@ -152,8 +171,16 @@ int launch_search(gastar_ctx* /*c: the current device's context*/, uint32_t kind
     lc.dynamicSmemBytes = smem;
     lc.stream = st;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = (P.team_ctas > 1 || P.n_heavy > 0) ? 1 : 0;
+    if (P.cluster) {  // a cluster's blocks are resident together by themselves
+        const uint32_t size = P.team_ctas > 1 ? P.team_ctas : P.heavy_team;
+        if (size > 8) GA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = (P.team_ctas > 1 || P.n_heavy > 0) ? 1 : 0;
+    }
     lc.attrs = attr;
     lc.numAttrs = 1;
     GA_CUDA(cudaLaunchKernelExC(&lc, f, args));
@@ -379,34 +406,85 @@ struct AttemptStats {
     uint64_t h2d = 0, d2h = 0;
 };
 
+struct PlainShape {
+    uint32_t ew = 0, W = 0;  // pops per warp-heap, warps per block
+    uint64_t blocks = 0;     // 0: no such shape
+    bool cluster = false;
+};
+
+// Shape of a ring team with the automatic widths: eight warps on every SM,
+// popping few entries each.  An iteration lasts as long as its slowest warp,
+// and a warp expands its pops in rounds (four grid cells, eight boards), so
+// many warps with one or two rounds beat fewer with more.  Measured: 16
+// 15-puzzles at Q = 16384 12.6 ms with 16-wide pops on 128 blocks, 10.5 with
+// 8-wide on 152 (4-wide: 13.0, too few pops); 1021^2 grid 11.3 ms with 16,
+// 9.2 with 8, 8.1 with 4; 4096^2 grid 49.5, 39.5 and 43.7 -- its frontier
+// (~4000 cells) fills 4-wide pops, hence the line at 2^22 cells.
+// Q above 16384 asks for throughput on hard puzzles: pops as wide as it says.
+static PlainShape ring_shape(const gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
+    PlainShape s;
+    const uint64_t warps = 8ull * (uint64_t)c->sms;
+    s.W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block) : 8u;
+    if (cfg.expansion_width) s.ew = std::min(32u, cfg.expansion_width);
+    else if (pp.kind == KIND_GRID) s.ew = (uint64_t)pp.W * pp.H >= (1ull << 22) ? 8 : 4;
+    else s.ew = (uint32_t)std::min<uint64_t>(Q <= 16384 ? 8 : 32, std::max<uint64_t>(4, (Q + warps - 1) / warps));
+    const bool fixed = cfg.expansion_width || cfg.warps_per_block;
+    const uint64_t heaps = std::min<uint64_t>((Q + s.ew - 1) / s.ew, fixed ? ~0ull : warps);
+    s.blocks = (heaps + s.W - 1) / s.W;
+    return s;
+}
+
+// Shape of a team that is one thread-block cluster (or one block), or none.
+// Up to 16 blocks pass their entries and minima through distributed shared
+// memory behind one cluster barrier (~400 cycles) instead of the ring's
+// fences and flags (~2400), but have a tenth of the SMs: taken for searches
+// whose iterations hold a few hundred entries -- Q that small, 8-puzzles
+// (181,440 states in all; 0.175 against 0.225 ms) and grids up to 2^17 cells
+// (200 x 150: 1.18 against 1.44 ms; 517 x 389: 3.94 against 3.66 ms).
+static PlainShape cluster_shape(const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
+    PlainShape s;
+    const bool fixed = cfg.expansion_width || cfg.warps_per_block;
+    s.W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block) : 8u;
+    s.ew = cfg.expansion_width ? std::min(32u, cfg.expansion_width) : 4u;
+    if (s.W > 8) return PlainShape();  // their kernel has no cluster teams for single instances
+    const bool few = pp.kind == KIND_SLIDING3 || (pp.kind == KIND_GRID && (uint64_t)pp.W * pp.H <= (1ull << 17));
+    uint64_t blocks = (Q + (uint64_t)s.ew * s.W - 1) / ((uint64_t)s.ew * s.W);
+    if (blocks > kMaxClusterBlocks) {
+        if (fixed || !few) return PlainShape();
+        blocks = kMaxClusterBlocks;
+    }
+    if (cfg.max_blocks) blocks = std::min<uint64_t>(blocks, cfg.max_blocks);
+    s.cluster = blocks > 1;
+    if (s.cluster) {
+        const uint32_t kinds = kind_bit(pp.kind);
+        const size_t smem = block_smem_bytes(kinds, s.W, s.ew, false, kHeapSmemNodes, cfg.open_list == 1);
+        if (occupancy_clusters(kinds, s.W * 32, smem, (uint32_t)blocks) < 1) return PlainShape();
+    }
+    s.blocks = blocks;
+    return s;
+}
+
 // Runs the search (+ path rebuild) once with the given capacities.
 static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg,
                          uint32_t table_log2, uint64_t heap_entries, std::vector<uint64_t>* path_keys,
                          cudaStream_t st, InstCtl& ctl_out, AttemptStats& as) {
     const bool want_path = path_keys != nullptr;
     const uint32_t kinds = kind_bit(pp.kind);
-    // Expansion width 0 = about 1024 warp-heaps per solve: wide enough pops
-    // for large Q, enough heaps (warps) to keep the SMs busy for small Q.
-    const uint32_t ew = cfg.expansion_width
-                            ? std::min(32u, cfg.expansion_width)
-                            : (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(8, (cfg.num_queues ? cfg.num_queues : 4096) / 1024));
     const uint64_t Q = cfg.num_queues ? cfg.num_queues : 4096;
-    uint64_t heaps = (Q + ew - 1) / ew;
-    // Warps per block 0 = 8 when that still gives at least half of the SMs a
-    // block (fewer, larger blocks: fewer parties to the hand-offs), else 4.
-    const uint32_t W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block)
-                                           : ((heaps / 8 >= (uint64_t)c->sms / 2) ? 8u : 4u);
-    const uint32_t threads = W * 32;
-    uint64_t blocks = (heaps + W - 1) / W;
-    const bool multi = blocks > 1;
+    PlainShape sh = cluster_shape(pp, cfg, Q);
+    if (!sh.blocks) sh = ring_shape(c, pp, cfg, Q);
+    const uint32_t ew = sh.ew, W = sh.W, threads = W * 32;
+    uint64_t blocks = sh.blocks, heaps = blocks * W;
+    const bool cluster = sh.cluster, multi = blocks > 1 && !cluster;  // multi: a ring team
     // Widening: a puzzle search with the automatic width that passes
     // kWideAfter iterations is a hard one, whose iteration count the pops per
     // iteration set rather than its depth; from then on every warp-heap pops
-    // twice as many (at most 32).  On the 64 15-puzzles of the plain
-    // benchmark (Q = 16384) the four hardest took 150-359 iterations and ran
-    // 1.3-1.4x faster with twice the pops, the rest at most ~90 iterations.
+    // four times as many (at most 32).  On the 64 15-puzzles of the plain
+    // benchmark (Q = 16384, 8-wide pops) the hardest took 333 iterations with
+    // twice the pops and takes 206 with four times; the 64 together 52.2 ->
+    // 50.3 ms.
     const uint32_t ew_wide =
-        multi && pp.kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 2 * ew) : ew;
+        multi && pp.kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 4 * ew) : ew;
     size_t smem = block_smem_bytes(kinds, W, ew, multi);
     const int nb = occupancy_blocks(c, kinds, threads, smem);
     if (nb <= 0) return GASTAR_CUDA_ERROR;
@@ -416,8 +494,12 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     // The shared memory the co-resident blocks leave free holds the heaps' top
     // levels: pops and pushes then touch global nodes only deep down.
     const bool buckets = cfg.open_list == 1;
-    const uint32_t snodes = fit_heap_snodes(c, kinds, W, ew, multi, threads,
+    uint32_t snodes = fit_heap_snodes(c, kinds, W, ew, multi, threads,
                                             (int)((blocks + c->sms - 1) / c->sms), &smem, buckets);
+    if (cluster && occupancy_clusters(kinds, threads, smem, (uint32_t)blocks) < 1) {
+        smem = block_smem_bytes(kinds, W, ew, multi, kHeapSmemNodes, buckets);
+        snodes = kHeapSmemNodes;
+    }
     if (multi && !c->coop) {
         set_error("device does not support cooperative launch");
         return GASTAR_CUDA_ERROR;
@@ -536,6 +618,7 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     P.team_ctas = (uint32_t)blocks;
     P.heap_snodes = snodes;
     P.buckets = buckets ? 1u : 0u;
+    P.cluster = cluster ? 1u : 0u;
     P.team = reinterpret_cast<TeamCtl*>(lb + kLbTeam);
     P.stage = c->stage.p;
     P.barrier_timeout_ns = 2000000000ull;

@@ -23,6 +23,13 @@ struct DevBuf {
 void set_error(const std::string& s);
 bool cuda_ok(cudaError_t e, const char* what);
 
+// The search kernel's instantiations (search_*.cu).
+const void* search_kernel_sliding3();
+const void* search_kernel_sliding4();
+const void* search_kernel_sliding5();
+const void* search_kernel_grid();
+const void* search_kernel_all();
+const void* search_kernel_all16();
 const void* search_kernel_for(uint32_t kinds, uint32_t threads);
 uint32_t entry_bytes(uint32_t kind);
 uint32_t max_neighbours(uint32_t kind);
@@ -43,6 +50,9 @@ int launch_paths(const InstDesc* d_insts, uint32_t n, unsigned long long* arena,
 uint32_t fit_heap_snodes(gastar_ctx* c, uint32_t kinds, uint32_t warps, uint32_t ew, bool multi, uint32_t threads,
                          int blocks_per_sm, size_t* smem, bool buckets = false);
 int occupancy_blocks(struct ::gastar_ctx* c, uint32_t kinds, uint32_t threads, size_t smem);
+// Clusters of `size` blocks of this shape that are resident at once (0: the
+// size or the shape does not fit).
+int occupancy_clusters(uint32_t kinds, uint32_t threads, size_t smem, uint32_t size);
 int device_min_weight(struct ::gastar_ctx* c, const uint8_t* d_w, uint64_t cells, cudaStream_t st,
                       uint32_t* out);
 // Places a grid's weights from the caller's host buffer at d_dst and returns

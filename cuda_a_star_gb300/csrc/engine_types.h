@@ -45,9 +45,10 @@ constexpr uint32_t kCuts = 16;  // cut slots in the ring (> 3 * kCutLag + 2)
 static_assert(kStageRing >= kCutLag + 2, "a stage buffer must be consumed before it is reused");
 
 constexpr uint32_t kMaxWarps = 16;  // warps of the largest block
+constexpr uint32_t kMaxClusterBlocks = 16;  // sizes above 8 need the opt-in attribute
 
 // Plain engine: iteration from which a puzzle search with the automatic
-// expansion width pops twice as many entries per warp-heap.
+// expansion width pops four times as many entries per warp-heap.
 constexpr uint32_t kWideAfter = 64;
 
 // Claim list: each warp reserves this many entries at a time; entries a warp
@@ -144,6 +145,7 @@ struct alignas(16) TeamSlot {
     uint32_t minstage;  // least f of the entries staged
     uint32_t best;      // goal costs found in the pop/expand phase
     uint32_t err;       // first error raised in the pop/expand phase
+    // The other blocks of a cluster read the two halves as 16 bytes each.
     uint32_t claims;    // table slots claimed
     uint32_t exps;      // entries expanded
     uint32_t minheap;   // least f over the heaps after the push phase
@@ -203,7 +205,7 @@ struct LaunchParams {
     uint32_t team_ctas;       // 1 = one block per instance; >1 = all blocks on instance 0
     uint32_t heap_snodes;     // shared-memory heap nodes per warp + 1 (0 = kHeapSmemNodes)
     uint32_t buckets;         // 1 = blocks carry the bucket push scratch (some instance has buckets)
-    uint32_t pad2;
+    uint32_t cluster;         // 1 = the blocks of a team are one thread-block cluster
     TeamCtl* team;            // multi-block team control (device)
     void* stage;              // multi-block stage buffer (device)
     uint64_t barrier_timeout_ns;

@@ -154,7 +154,7 @@ extern "C" int gastar_solve_sliding_noalloc(uint32_t n, const uint8_t* start, co
     if ((e = cudaMemsetAsync(b + kCtlOff, 0, kHdrOff - kCtlOff, st)) != cudaSuccess)
         return fail(e, "cudaMemsetAsync");
     out->h2d_bytes = sizeof(d);
-    const void* kern = reinterpret_cast<const void*>(&search_kernel<kind_bit(KIND_SLIDING3)>);
+    const void* kern = search_kernel_for(kind_bit(KIND_SLIDING3), kWarps * 32);
     void* args[] = {&P};
     const size_t smem = 2 * stage_entries_per_buffer(kWarps, kEw, 4) * 16 + (size_t)kWarps * (kHeapSmemNodes - 1) * 32 * 16;
     if ((e = cudaLaunchKernel(kern, dim3(1), dim3(kWarps * 32), args, smem, st)) != cudaSuccess)

@@ -203,8 +203,13 @@ struct PluginDom {
     }
     static __device__ __forceinline__ bool is_goal(const Ctx& c, const KeyT& k) { return k == c.goal; }
     static __device__ __forceinline__ bool is_start(const Ctx& c, const KeyT& k) { return k == c.start; }
-    static __device__ __forceinline__ bool succ(const Ctx&, const KeyT& k, int m, uint32_t g, uint32_t, KeyT& nk,
-                                                uint32_t& ng, uint32_t& nh) {
+    struct Move {};
+    static __device__ __forceinline__ Move lane_move(const Ctx&, int) { return Move(); }
+    static __device__ __forceinline__ uint32_t tag(int m, const KeyT&, uint32_t) { return (uint32_t)m; }
+    static __device__ __forceinline__ uint32_t start_tag(const KeyT&) { return kRootMove; }
+    static __device__ __forceinline__ bool succ(const Ctx&, const Move&, int m, const KeyT& k, uint32_t, uint32_t g,
+                                                uint32_t, KeyT& nk, uint32_t& ng, uint32_t& nh, uint32_t& at) {
+        at = 0;
         const T src = from_key(k);
         T dst = src;
         bool ex = false;

@@ -9,15 +9,16 @@
 //            successors, computes g and an incrementally updated h, and does
 //            one insert-or-min on the duplicate-detection table per
 //            successor; improved successors go to the block's stage area;
-//   push   : one-block teams deal their stage chunks round-robin (rotating
-//            offset) to their warps after a block barrier; in a multi-block
-//            team block c pushes the stage region of block (c + i) mod blocks
-//            once that block has flagged it ready (no team barrier);
+//   push   : one-block and cluster teams deal their stage chunks round-robin
+//            (rotating offset) to their warps after a barrier, a cluster's
+//            through distributed shared memory; in a ring team block c pushes
+//            the stage region of block (c + i) mod blocks once that block has
+//            flagged it ready (no team barrier);
 //   check  : the search ends when the best goal cost is <= min f over all
-//            open entries -- over the block's slots (one-block teams) or over
-//            the cut every block publishes with its stage region, one
-//            hand-off per iteration (multi-block teams, tested kCutLag
-//            iterations later).
+//            open entries -- over the blocks' slots (one block, cluster) or
+//            over the cut every block publishes with its stage region, one
+//            hand-off per iteration (ring teams, tested kCutLag iterations
+//            later).
 // This is the reference's iteration (a_star.h:247-264: extract_nodes, three
 // bitonic sorts, mark_duplicates, insert_unique_data, remove_updated_elements,
 // insert_nodes_into_queues, two host reductions) as one device-resident loop
@@ -160,31 +161,43 @@ template <int N> struct SlidingDom {
     }
     static __device__ __forceinline__ bool is_goal(const Ctx& c, KeyT k) { return k == c.goal; }
     static __device__ __forceinline__ bool is_start(const Ctx& c, KeyT k) { return k == c.start; }
-    // Whether move m leads straight back to the parent reached with move pm.
-    static __device__ __forceinline__ bool is_back(int m, uint32_t pm) { return (uint32_t)(m ^ 1) == pm; }
+    // Low byte of an entry's priority word: the blank's cell and the move the
+    // entry was reached with (4: the start), so that an expansion neither
+    // searches the board for the blank nor looks its parent up.
+    static __device__ __forceinline__ uint32_t tag(int m, KeyT nk, uint32_t cell) { return cell << 3 | (uint32_t)m; }
+    static __device__ __forceinline__ uint32_t start_tag(KeyT k) { return tag(4, k, (uint32_t)blank_of(k)); }
+    // Whether move m leads straight back to the parent of an entry with this tag.
+    static __device__ __forceinline__ bool is_back(int m, uint32_t tag) { return (uint32_t)(m ^ 1) == (tag & 7u); }
+    // What a lane's move does, fixed for a search: the shift of the blank's
+    // cell and the cells it is possible from.
+    struct Move {
+        int dq;
+        uint32_t from;
+    };
+    static __device__ __forceinline__ Move lane_move(const Ctx& c, int m) {
+        constexpr uint32_t all = (1u << C) - 1u, row = (1u << N) - 1u;
+        uint32_t left = 0;  // cells of the first column
+#pragma unroll
+        for (int i = 0; i < N; ++i) left |= 1u << (i * N);
+        Move v;
+        v.dq = m == 0 ? N : m == 1 ? -N : m == 2 ? 1 : -1;
+        v.from = m == 0 ? all & ~(row << (C - N)) : m == 1 ? all & ~row : m == 2 ? all & ~(left << (N - 1)) : all & ~left;
+        if (m >= 4 || (c.ref_moves && (m & 1))) v.from = 0;  // the reference's moves 1 and 3 never exist
+        return v;
+    }
 
-    static __device__ __forceinline__ bool succ(const Ctx& c, KeyT k, int m, uint32_t g, uint32_t h, KeyT& nk,
-                                                uint32_t& ng, uint32_t& nh) {
-        const int p = blank_of(k), r = p / N, col = p % N;
-        int q;
-        if (m == 0) {
-            if (r >= N - 1) return false;
-            q = p + N;
-        } else if (m == 1) {
-            if (c.ref_moves || r == 0) return false;
-            q = p - N;
-        } else if (m == 2) {
-            if (col >= N - 1) return false;
-            q = p + 1;
-        } else {
-            if (c.ref_moves || col == 0) return false;
-            q = p - 1;
-        }
+    // The successor by a lane's move: the tile at the new blank cell q slides
+    // to the old one p (whose field is zero).  `at` becomes q.
+    static __device__ __forceinline__ bool succ(const Ctx& c, const Move& mv, int, KeyT k, uint32_t tag, uint32_t g,
+                                                uint32_t h, KeyT& nk, uint32_t& ng, uint32_t& nh, uint32_t& at) {
+        const int p = (int)(tag >> 3), q = p + mv.dq;
+        if (!(mv.from >> p & 1u)) return false;
         const uint32_t t = field(k, q);
-        nk = (k & ~(KeyT((1u << B) - 1) << (B * q))) | (KeyT(t) << (B * p));
+        nk = k ^ (KeyT(t) << (B * q)) ^ (KeyT(t) << (B * p));
         nh = h + c.md[t][p] - c.md[t][q];
         if (c.ref_h) nh = nh + c.md[0][q] - c.md[0][p];
         ng = g + 1;
+        at = (uint32_t)q;
         return true;
     }
 
@@ -264,8 +277,22 @@ struct GridDom {
         return old == kEmpty ? 1 : 0;
     }
     static __device__ __forceinline__ bool is_goal(const Ctx& c, KeyT k) { return (uint32_t)k == c.goal; }
-    static __device__ __forceinline__ bool is_back(int m, uint32_t pm) {
-        return pm != kRootMove && (uint32_t)m == inv(pm);
+    // Low byte of an entry's priority word: the move it was reached with.
+    static __device__ __forceinline__ uint32_t tag(int m, KeyT, uint32_t) { return (uint32_t)m; }
+    static __device__ __forceinline__ uint32_t start_tag(KeyT) { return kRootMove; }
+    static __device__ __forceinline__ bool is_back(int m, uint32_t tag) {
+        return tag != kRootMove && (uint32_t)m == inv(tag);
+    }
+    // What a lane's move does, fixed for a search.
+    struct Move {
+        int dx, dy, dcell;
+    };
+    static __device__ __forceinline__ Move lane_move(const Ctx& c, int m) {
+        Move v;
+        v.dx = (int)((kGridDxPack >> (2 * m)) & 3u) - 1;
+        v.dy = (int)((kGridDyPack >> (2 * m)) & 3u) - 1;
+        v.dcell = v.dy * (int)c.W + v.dx;
+        return v;
     }
     static __device__ __forceinline__ uint32_t heur(const Ctx& c, int x, int y) {
         // 0: Chebyshev x min weight (admissible); 1: Manhattan (the reference's,
@@ -275,12 +302,11 @@ struct GridDom {
         if (c.href == 2) return 0;
         return (ax > ay ? ax : ay) * c.minw;
     }
-    // The cell move m enters from k and its h; false off the board.
-    static __device__ __forceinline__ bool step(const Ctx& c, KeyT k, int m, KeyT& nk, uint32_t& nh) {
-        const int ddx = (int)((kGridDxPack >> (2 * m)) & 3u) - 1, ddy = (int)((kGridDyPack >> (2 * m)) & 3u) - 1;
-        const int nx = (int)(uint32_t)(k >> 32 & 0xffffu) + ddx, ny = (int)(uint32_t)(k >> 48) + ddy;
+    // The cell a lane's move enters from k and its h; false off the board.
+    static __device__ __forceinline__ bool step(const Ctx& c, const Move& mv, KeyT k, KeyT& nk, uint32_t& nh) {
+        const int nx = (int)((uint32_t)(k >> 32) & 0xffffu) + mv.dx, ny = (int)(uint32_t)(k >> 48) + mv.dy;
         if ((uint32_t)nx >= c.W || (uint32_t)ny >= c.H) return false;
-        nk = make_key((uint32_t)k + (uint32_t)(ddy * (int)c.W + ddx), (uint32_t)nx, (uint32_t)ny);
+        nk = make_key((uint32_t)k + (uint32_t)mv.dcell, (uint32_t)nx, (uint32_t)ny);
         nh = heur(c, nx, ny);
         return true;
     }
@@ -300,8 +326,12 @@ struct CtaShared {
     unsigned long long wcnt[kMaxWarps][3];  // per warp: stale, generated, pushed in this launch
     unsigned long long t_start;  // search start on the device clock
     uint32_t dec_status, dec_best, dec_fmin, push_count;  // thread 0 -> block
+    // Cluster teams, warp 0 -> block: best, error, least open f, chunks in
+    // all, entries per chunk; per block the chunks before its own, its entries.
+    uint32_t plan[8], plan_before[kMaxClusterBlocks], plan_count[kMaxClusterBlocks];
     InstDesc desc;
-    uint32_t inst, ok, slice, pad1;  // slice: iterations before suspending (0 = to the end)
+    alignas(16) uint32_t inst;
+    uint32_t ok, slice, pad1;  // slice: iterations before suspending (0 = to the end)
     union {
         SlidingDom<3>::Ctx s3;
         SlidingDom<4>::Ctx s4;
@@ -471,21 +501,50 @@ template <int LPE> __device__ constexpr uint32_t group_mask() {
 }
 
 
-// How the blocks of a team work together.
-enum TeamKind : int { TEAM_BLOCK, TEAM_RING };
+// How the blocks of a team work together: one block; the blocks of one
+// thread-block cluster, through each other's shared memory; any number of
+// blocks, through a ring of stage buffers in global memory.
+enum TeamKind : int { TEAM_BLOCK, TEAM_CLUSTER, TEAM_RING };
+
+// Barrier over the cluster's blocks; orders their shared and global memory.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// 16 bytes at shared-memory address `p` of the cluster's block `rank`.
+__device__ __forceinline__ uint4 ld_cluster(const void* p, uint32_t rank) {
+    uint4 v;
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("{\n\t.reg .u32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\t"
+                 "ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [ra];\n\t}"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(a), "r"(rank)
+                 : "memory");
+    return v;
+}
+template <int KW> __device__ __forceinline__ Entry<KW> ld_stage_cluster(const Entry<KW>* p, uint32_t rank) {
+    Entry<KW> e;
+#pragma unroll
+    for (int v = 0; v < entry_vecs<KW>(); ++v) {
+        const uint4 a = ld_cluster(reinterpret_cast<const uint4*>(p) + v, rank);
+        set_word(e, 2 * v, (uint64_t(a.y) << 32) | a.x);
+        set_word(e, 2 * v + 1, (uint64_t(a.w) << 32) | a.z);
+    }
+    return e;
+}
 
 template <class D, int MAXT, int TEAM>
 __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef tm) {
     constexpr int KW = D::KW;
     constexpr int MAXN = D::MAXN;
-    constexpr bool multi = TEAM == TEAM_RING;
+    constexpr bool ring = TEAM == TEAM_RING, cluster = TEAM == TEAM_CLUSTER;
+    constexpr bool multi = ring || cluster;  // several blocks
     using E = Entry<KW>;
     using KeyT = typename D::KeyT;
     constexpr int LPE = lanes_per_entry(MAXN);  // lanes per entry: one per move
     constexpr int EPR = 32 / LPE;               // entries per expansion round
-    // Rounds whose probes are in flight together (registers: 16-warp blocks
-    // have 128 per thread, and twice the warps to overlap).
-    constexpr int RB = KW == 1 && MAXT <= 256 ? 4 : 2;
+    // Rounds whose probes are in flight together.  Blocks of 9 to 16 warps
+    // have 128 registers per thread and overlap their warps' rounds instead.
+    constexpr int RB = MAXT > 256 ? 1 : KW == 1 ? 4 : 2;
     CtaShared& sm = cta();
     const InstDesc& d = sm.desc;
     typename D::Ctx& ctx = shared_ctx<D>();
@@ -494,15 +553,16 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
     InstCtl* const ctl = d.ctl;
     const bool leader = rank == 0 && threadIdx.x == 0;
     const uint32_t hid = rank * W + warp;
-    // One-block teams stage in shared memory (two buffers), multi-block teams
-    // in a global ring.
+    // Blocks and clusters stage in shared memory (two buffers), ring teams in
+    // global memory.
     const uint32_t region_cap =
         (uint32_t)stage_entries_per_buffer(W, d.ew_wide > d.ew ? d.ew_wide : d.ew, MAXN);  // widest pop of the search
-    E* const snodes_all = reinterpret_cast<E*>(g_dyn_smem) + (multi ? 0u : 2 * region_cap);
+    E* const snodes_all = reinterpret_cast<E*>(g_dyn_smem) + (ring ? 0u : 2 * region_cap);
 
     auto tsync = [&]() -> bool {
-        if constexpr (multi) return team_sync_grid(tm.ctl, tm.ctas, P.barrier_timeout_ns);
-        __syncthreads();
+        if constexpr (ring) return team_sync_grid(tm.ctl, tm.ctas, P.barrier_timeout_ns);
+        if constexpr (cluster) cluster_sync();
+        else __syncthreads();
         return true;
     };
 
@@ -531,7 +591,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
     bq_init(bq, lane);
 
     const uint32_t life = uniform(ld_vol(&ctl->life));
-    if (!multi && threadIdx.x < kSlots) slot_clear(sm.slot[threadIdx.x]);
+    if (!ring && threadIdx.x < kSlots) slot_clear(sm.slot[threadIdx.x]);
     if (lane < 3) sm.wcnt[warp][lane] = 0;
     uint32_t status = kInf;  // kInf while running / suspended
     uint32_t best_r;         // best goal cost seen (identical in every thread)
@@ -562,15 +622,13 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             if ((d.table_words & 1) && tid == 0)  // odd cell count: last word
                 __stcg(d.table + d.table_words - 1, kEmpty);
         }
-        heap_init(hp, lane);
+        heap_init(hp);
         if (!tsync()) status = ST_BARRIER;
         if (hid == 0) {
             E s = inf_entry<KW>();
-            s.prio = make_prio(D::start_f(ctx, d), 0, kRootMove);
+            s.prio = make_prio(D::start_f(ctx, d), 0, D::start_tag(ctx.start));
             D::set_key(s, ctx.start);
-            if (lane == 0) st_part(hp, 0, s);
-            __syncwarp();
-            hp.pc = 1;
+            heap_push(hp, lane == 0 ? s : inf_entry<KW>(), 1u, lane);
         }
         if (leader) {
             uint64_t old;
@@ -591,13 +649,13 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         best_r = uniform(ld_vol(&ctl->best));
         have_prev = false;
     }
-    // Multi-block teams: each block stages into its own region of the ring
+    // Ring teams: each block stages into its own region of the ring
     // buffers and aggregates its counters and minima in shared memory; thread
     // 0 publishes them (ready word, cut slot).
-    E* const stage0 = multi ? reinterpret_cast<E*>(tm.stage) : reinterpret_cast<E*>(g_dyn_smem);
+    E* const stage0 = ring ? reinterpret_cast<E*>(tm.stage) : reinterpret_cast<E*>(g_dyn_smem);
     unsigned long long* const ready =
-        multi ? reinterpret_cast<unsigned long long*>(stage0 + (size_t)kStageRing * tm.ctas * region_cap) : nullptr;
-    if (multi && threadIdx.x == 0) {
+        ring ? reinterpret_cast<unsigned long long*>(stage0 + (size_t)kStageRing * tm.ctas * region_cap) : nullptr;
+    if (ring && threadIdx.x == 0) {
         for (uint32_t r = 0; r < kStageRing; ++r) ready[(size_t)r * tm.ctas + rank] = 0;
         if (rank == 0)
             for (uint32_t k = 0; k < kCuts; ++k) {
@@ -610,6 +668,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
     }
     if (status == kInf && !tsync()) status = ST_BARRIER;
 
+    const int sub = lane & (LPE - 1);
+    const typename D::Move mv = D::lane_move(ctx, sub);
     // This warp's current claim-list chunk (none reserved yet).
     unsigned long long t_base = 0;
     uint32_t t_used = kTouchedChunk;
@@ -628,29 +688,31 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         sm.run[0] = sm.run[1] = sm.mine[0] = sm.mine[1] = 0;
     }
     __syncthreads();
-    // The first cut of a multi-block team holds the heaps as they are now.
-    if (multi) {
+    // The first cut of a ring team holds the heaps as they are now.
+    if (ring) {
         const uint32_t mf = open_minf(hp, bq);
         if (lane == 0 && mf != kInf) atomicMin(&sm.agg_minheap, mf);
     }
     while (status == kInf) {
         TeamSlot* const S = &sm.slot[it % kSlots];
-        // Where this block's warps record the iteration: the team slot itself
-        // for one-block teams (shared memory), the block aggregate otherwise.
-        TeamSlot* const Sw = multi ? &sm.agg : S;
-        E* const stage = multi ? stage0 + ((size_t)(it % kStageRing) * tm.ctas + rank) * region_cap
+        // Where this block's warps record the iteration: its slot, or for ring
+        // teams the block aggregate.
+        TeamSlot* const Sw = ring ? &sm.agg : S;
+        E* const stage = ring ? stage0 + ((size_t)(it % kStageRing) * tm.ctas + rank) * region_cap
                                : reinterpret_cast<E*>(g_dyn_smem) + (it & 1) * region_cap;
         const typename D::Tab tab = D::make_tab(d);
-        if (!multi && leader) {
-            // One-block team: slot it+1 was last read right after the block
-            // barrier of iteration it-2; every warp is past that point, and
-            // none writes it before the barrier of this iteration.
+        if (!ring && threadIdx.x == 0) {
+            // Slot it+1 was last read right after the barrier of iteration
+            // it-2; every warp is past that point, and none writes it before
+            // the barrier of this iteration.
             slot_clear(sm.slot[(it + 1) % kSlots]);
-            if (it) {  // the previous iteration's counts are complete
+            if (!cluster && it) {  // the previous iteration's counts are complete
                 const TeamSlot& pv = sm.slot[(it + kSlots - 1) % kSlots];
                 sm.run[0] += pv.claims;
                 sm.run[1] += pv.exps;
             }
+        }
+        if (!ring && leader) {
             if (sm.base[0] + sm.run[0] > d.table_limit) atomicCAS(&S->err, 0u, (uint32_t)ST_TABLE_FULL);
             if (d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
             if (d.max_iter && it0 + it + 1 >= d.max_iter) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
@@ -706,9 +768,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         // branches to the compiler too.
         const uint32_t popped = __ballot_sync(kFull, (uint32_t)lane < cnt);
         const uint32_t lt = (1u << lane) - 1u;
-        const int sub = lane & (LPE - 1);
         uint32_t n_gen = 0, n_claim = 0, pushed = 0, fstage = kInf;
-        bool tfull = false, range = false;
+        uint32_t flags = 0;  // 1: the table is full, 2: a cost out of range
         for (uint32_t r0 = 0; r0 < (uint32_t)LPE && (popped >> (r0 * EPR)) != 0; r0 += RB) {
 #pragma unroll 1
             for (int mg = 0; mg < MAXN; mg += LPE) {
@@ -718,6 +779,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 uint64_t old[RB], seen[RB], own_v[RB];
                 uint32_t slot[RB];
                 uint32_t code[RB];  // parent as recorded in the table
+                uint32_t at[RB];    // puzzles: the blank's cell
                 bool ok[RB], own[RB];
                 // Issue: nothing here waits for a probe, so RB rounds' probes
                 // are in flight together.
@@ -728,27 +790,28 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                     const int src = (int)((r0 + j) * EPR) + lane / LPE;
                     const E x = shfl_idx(e, src);
                     const KeyT xk = D::key_of(x);
-                    const uint32_t xg = prio_g(x.prio), pm = prio_pm(x.prio);
+                    const uint32_t xg = prio_g(x.prio), tag = prio_pm(x.prio);
                     uint32_t xself = 0, nh = 0;
                     if constexpr (D::kParentBySlot) xself = __shfl_sync(kFull, self, src);
                     const bool on = ((live >> src) & 1u) && m < MAXN;
-                    if constexpr (!D::kParentBySlot) own[j] = on && D::is_back(m, pm);
+                    if constexpr (!D::kParentBySlot) own[j] = on && D::is_back(m, tag);
                     ng[j] = xg;
                     if constexpr (D::kDense) {
                         // The neighbour's weight and value load together; a
                         // value that is already as good needs no atomic
                         // (four of five do not: 7.5 M of 9.8 M generated on
                         // a 1021^2 grid), and a load costs half an atomic.
-                        ok[j] = on && !own[j] && D::step(ctx, xk, m, nk[j], nh);
+                        ok[j] = on && !own[j] && D::step(ctx, mv, xk, nk[j], nh);
                         if (own[j]) nk[j] = xk;
                         if (ok[j] || own[j]) old[j] = D::get(tab, nk[j]);
                         if (ok[j]) wt[j] = D::weight(ctx, nk[j]);
                         nf[j] = nh;
                     } else {
-                        ok[j] = on && !own[j] && D::succ(ctx, xk, m, xg, prio_f(x.prio) - xg, nk[j], ng[j], nh);
+                        ok[j] = on && !own[j] &&
+                                D::succ(ctx, mv, m, xk, tag, xg, prio_f(x.prio) - xg, nk[j], ng[j], nh, at[j]);
                         n_gen += __popc(__ballot_sync(kFull, ok[j]));
                         if (ok[j] && ng[j] > kMaxG) {
-                            range = true;
+                            flags |= 2u;
                             ok[j] = false;
                         }
                         nf[j] = ng[j] + nh;
@@ -775,7 +838,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                         n_gen += __popc(__ballot_sync(kFull, ok[j]));
                         if (ok[j]) ng[j] += wt[j];
                         if (ok[j] && ng[j] > kMaxG) {
-                            range = true;
+                            flags |= 2u;
                             ok[j] = false;
                         }
                         nf[j] += ng[j];
@@ -797,7 +860,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                     } else {
                         if (ok[j]) cl = D::claim_end(tab, nk[j], make_val(ng[j], code[j]), slot[j], seen[j],
                                                      old[j]);
-                        if (ok[j] && cl < 0) tfull = true;
+                        if (ok[j] && cl < 0) flags |= 1u;
                         if constexpr (!D::kParentBySlot) {
                             // A stale entry's successors are real paths and
                             // stay in the table, but are not queued; the
@@ -832,9 +895,9 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                     for (int j = 0; j < RB; ++j) {
                         if (acc_at[j] != kInf) {
                             E out = inf_entry<KW>();
-                            out.prio = make_prio(nf[j], ng[j], (uint32_t)m);
+                            out.prio = make_prio(nf[j], ng[j], D::tag(m, nk[j], D::kDense ? 0u : at[j]));
                             D::set_key(out, nk[j]);
-                            st_stage<multi>(stage + base + acc_at[j], out);
+                            st_stage<ring>(stage + base + acc_at[j], out);
                         }
                     }
                 }
@@ -864,13 +927,14 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 }
             }
         }
-        __syncwarp();
         {
             // The counts are warp-uniform; minima over the lanes with one
             // reduction each.
             const uint32_t smin = __reduce_min_sync(kFull, fstage);
             goal_g = __reduce_min_sync(kFull, goal_g);
-            const bool any_full = __any_sync(kFull, tfull), any_range = __any_sync(kFull, range);
+            // One reduction for both flags.  (Not a vote each: the first is a
+            // constant for grids, and a vote on a constant here hung the warp.)
+            flags = uniform(flags);
             if (lane == 0) {
                 const uint32_t n_exp = __popc(live) - (D::kParentBySlot ? 0u : n_stale);
                 sm.wcnt[warp][0] += n_stale;
@@ -880,12 +944,11 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 if (n_claim) atomicAdd(&Sw->claims, n_claim);
                 if (smin != kInf) atomicMin(&Sw->minstage, smin);
                 if (goal_g != kInf) atomicMin(&Sw->best, goal_g);
-                if (any_full) atomicCAS(&Sw->err, 0u, (uint32_t)ST_TABLE_FULL);
-                if (any_range) atomicCAS(&Sw->err, 0u, (uint32_t)ST_COST_RANGE);
+                if (flags & 1u) atomicCAS(&Sw->err, 0u, (uint32_t)ST_TABLE_FULL);
+                if (flags & 2u) atomicCAS(&Sw->err, 0u, (uint32_t)ST_COST_RANGE);
             }
-            __syncwarp();
         }
-        if constexpr (multi) {
+        if constexpr (ring) {
             // ---- one hand-off per iteration: publish cut `it` and this
             // block's stage region, then wait for the region this block
             // pushes and test cut it - kCutLag (a_star.h:260-262) ----
@@ -987,16 +1050,77 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             // ---- termination test (a_star.h:260-262), one iteration behind ----
             // Open entries now: heaps after the previous push (>= that slot's
             // min) minus this iteration's pops, plus this iteration's stage.
-            const uint32_t sb = uniform(ld_vol(&S->best));
-            best_r = sb < best_r ? sb : best_r;
-            uint32_t err = uniform(ld_vol(&S->err));
-            uint32_t open_f = uniform(ld_vol(&S->minstage));
-            if (have_prev) {
-                const TeamSlot* pv = &sm.slot[(it + kSlots - 1) % kSlots];
-                const uint32_t pe = uniform(ld_vol(&pv->perr)), mf = uniform(ld_vol(&pv->minheap));
-                if (!err) err = pe;
-                open_f = mf < open_f ? mf : open_f;
+            const TeamSlot* pv = &sm.slot[(it + kSlots - 1) % kSlots];
+            uint32_t err, open_f, sb;
+            if constexpr (cluster) {
+                // One warp per block reads the blocks' slots through
+                // distributed shared memory (lane j block j's), reduces them
+                // and plans the push; the others wait for its record (all
+                // warps reading all slots took no less, 1.5 k cycles).
+                if (warp == 0) {
+                    uint4 a = make_uint4(0, kInf, kInf, 0), q = make_uint4(0, 0, kInf, 0);
+                    uint2 n = make_uint2(0, 0);
+                    if ((uint32_t)lane < tm.ctas) {
+                        a = ld_cluster(&S->count, (uint32_t)lane);
+                        q = ld_cluster(&pv->claims, (uint32_t)lane);
+                        if (rank == 0) {
+                            const uint4 c = ld_cluster(&S->claims, (uint32_t)lane);
+                            n = make_uint2(c.x, c.y);
+                        }
+                    }
+                    if (!have_prev) q.z = kInf, q.w = 0;
+                    const uint32_t b_min = __reduce_min_sync(kFull, a.z);
+                    // The largest code wins: lost entries before budgets.
+                    const uint32_t e_max = __reduce_max_sync(kFull, a.w > q.w ? a.w : q.w);
+                    const uint32_t f_min = __reduce_min_sync(kFull, a.y < q.z ? a.y : q.z);
+                    if (rank == 0) {  // the team's counts, for the budgets
+                        const uint32_t nc = __reduce_add_sync(kFull, n.x), ne = __reduce_add_sync(kFull, n.y);
+                        if (lane == 0) {
+                            sm.run[0] += nc;
+                            sm.run[1] += ne;
+                        }
+                    }
+                    const uint32_t NW = tm.ctas * (uint32_t)W;
+                    const uint32_t total = __reduce_add_sync(kFull, a.x);
+                    // A block's last chunk may be short: a chunk of slack per
+                    // block keeps the chunks at one per warp.
+                    const uint32_t room = W > 1 ? NW - tm.ctas : NW;
+                    const uint32_t per = (total + room - 1) / room;
+                    const uint32_t cs = per < 32 ? (per ? per : 1u) : 32u;
+                    const uint32_t chunks = (a.x + cs - 1) / cs;
+                    uint32_t upto = chunks;  // chunks of blocks 0..lane
+#pragma unroll
+                    for (int o = 1; o < (int)kMaxClusterBlocks; o <<= 1) {
+                        const uint32_t t = __shfl_up_sync(kFull, upto, o);
+                        if (lane >= o) upto += t;
+                    }
+                    if (lane < (int)kMaxClusterBlocks) {
+                        sm.plan_before[lane] = upto - chunks;
+                        sm.plan_count[lane] = a.x;
+                    }
+                    if (lane == (int)kMaxClusterBlocks - 1) {
+                        sm.plan[0] = b_min;
+                        sm.plan[1] = e_max;
+                        sm.plan[2] = f_min;
+                        sm.plan[3] = upto;
+                        sm.plan[4] = cs;
+                    }
+                }
+                __syncthreads();
+                sb = uniform(ld_vol(&sm.plan[0]));
+                err = uniform(ld_vol(&sm.plan[1]));
+                open_f = uniform(ld_vol(&sm.plan[2]));
+            } else {
+                sb = uniform(ld_vol(&S->best));
+                err = uniform(ld_vol(&S->err));
+                open_f = uniform(ld_vol(&S->minstage));
+                if (have_prev) {
+                    const uint32_t pe = uniform(ld_vol(&pv->perr)), mf = uniform(ld_vol(&pv->minheap));
+                    if (!err) err = pe;
+                    open_f = mf < open_f ? mf : open_f;
+                }
             }
+            best_r = sb < best_r ? sb : best_r;
             // An iteration that lost entries (full table or heap) proves nothing.
             if (err == ST_TABLE_FULL || err == ST_HEAP_FULL || err == ST_COST_RANGE) status = err;
             else if (have_prev && best_r != kInf && best_r <= open_f) status = ST_OK;
@@ -1008,44 +1132,61 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
 
         // ---- push ----
         // One-block teams deal the block's stage chunks round-robin with a
-        // rotating offset; in a multi-block team block r takes the region of
-        // block (r + it) mod blocks, so work moves between blocks every
-        // iteration, and its warps deal that region's chunks.
+        // rotating offset; cluster teams deal all blocks' chunks the same way
+        // over all of the cluster's warps; in a ring team block r takes the
+        // region of block (r + it) mod blocks, so work moves between blocks
+        // every iteration, and its warps deal that region's chunks.
+        // Chunks hold up to 32 entries, fewer when that gives every warp a
+        // share: a warp expands its pops in rounds.
         {
-            uint32_t total;
-            const E* src;
-            uint32_t first, step;
-            if constexpr (multi) {
-                const uint32_t from = (rank + it) % tm.ctas;
-                total = uniform(sm.push_count);
-                src = stage0 + ((size_t)(it % kStageRing) * tm.ctas + from) * region_cap;
-                first = ((uint32_t)warp + it) % (uint32_t)W;
-                step = (uint32_t)W;
-            } else {
-                total = uniform(ld_vol(&S->count));
-                src = stage;
-                first = ((uint32_t)warp + (uint32_t)W - it % (uint32_t)W) % (uint32_t)W;
-                step = (uint32_t)W;
-            }
-            // Chunks of up to 32 entries, smaller when that gives every warp
-            // of the block a share: a warp expands its pops in rounds.
-            const uint32_t per = (total + (uint32_t)W - 1) / (uint32_t)W;
-            const uint32_t cs = per < 32 ? per : 32u;
-            const uint32_t nch = cs ? (total + cs - 1) / cs : 0u;
             bool hfull = false;
-            for (uint32_t c = first; c < nch; c += step) {
-                const uint32_t idx = c * cs + (uint32_t)lane;
-                const uint32_t m = total - c * cs < cs ? total - c * cs : cs;
-                E x = (uint32_t)lane < m ? ld_stage<multi>(src + idx) : inf_entry<KW>();
-                if (!open_push(hp, bq, x, m, lane)) {
-                    hfull = true;
-                    break;
+            if constexpr (cluster) {
+                const uint32_t NW = tm.ctas * (uint32_t)W;
+                const uint32_t nch = uniform(ld_vol(&sm.plan[3])), cs = uniform(ld_vol(&sm.plan[4]));
+                for (uint32_t c = (hid + NW - it % NW) % NW; c < nch; c += NW) {
+                    // The block whose chunks c falls among.
+                    const uint32_t before = lane < (int)kMaxClusterBlocks ? ld_vol(&sm.plan_before[lane]) : kInf;
+                    const uint32_t from = 31 - __clz(__ballot_sync(kFull, (uint32_t)lane < tm.ctas && before <= c));
+                    const uint32_t at = (c - uniform(ld_vol(&sm.plan_before[from]))) * cs;
+                    const uint32_t left = uniform(ld_vol(&sm.plan_count[from])) - at;
+                    const uint32_t m = left < cs ? left : cs;
+                    const E x = (uint32_t)lane < m ? ld_stage_cluster(stage + at + lane, from) : inf_entry<KW>();
+                    if (!open_push(hp, bq, x, m, lane)) {
+                        hfull = true;
+                        break;
+                    }
+                }
+            } else {
+                uint32_t total;
+                const E* src;
+                uint32_t first;
+                if constexpr (ring) {
+                    const uint32_t from = (rank + it) % tm.ctas;
+                    total = uniform(sm.push_count);
+                    src = stage0 + ((size_t)(it % kStageRing) * tm.ctas + from) * region_cap;
+                    first = ((uint32_t)warp + it) % (uint32_t)W;
+                } else {
+                    total = uniform(ld_vol(&S->count));
+                    src = stage;
+                    first = ((uint32_t)warp + (uint32_t)W - it % (uint32_t)W) % (uint32_t)W;
+                }
+                const uint32_t per = (total + (uint32_t)W - 1) / (uint32_t)W;
+                const uint32_t cs = per < 32 ? per : 32u;
+                const uint32_t nch = cs ? (total + cs - 1) / cs : 0u;
+                for (uint32_t c = first; c < nch; c += (uint32_t)W) {
+                    const uint32_t idx = c * cs + (uint32_t)lane;
+                    const uint32_t m = total - c * cs < cs ? total - c * cs : cs;
+                    E x = (uint32_t)lane < m ? ld_stage<ring>(src + idx) : inf_entry<KW>();
+                    if (!open_push(hp, bq, x, m, lane)) {
+                        hfull = true;
+                        break;
+                    }
                 }
             }
             const uint32_t mf = open_minf(hp, bq);
             if (lane == 0) {
-                atomicMin(multi ? &sm.agg_minheap : &S->minheap, mf);
-                if (hfull) atomicCAS(multi ? &sm.agg_err_prev : &S->perr, 0u, (uint32_t)ST_HEAP_FULL);
+                atomicMin(ring ? &sm.agg_minheap : &S->minheap, mf);
+                if (hfull) atomicCAS(ring ? &sm.agg_err_prev : &S->perr, 0u, (uint32_t)ST_HEAP_FULL);
             }
         }
         ++it;
@@ -1058,9 +1199,15 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         for (uint32_t i = t_used + (uint32_t)lane; i < kTouchedChunk; i += 32)
             if (t_base + i < d.touched_cap) d.touched[t_base + i] = kTouchedHole;
     {  // this launch's counters
-        __syncthreads();
+        if constexpr (cluster) cluster_sync();  // no block reads another's slots or stage any more
+        else __syncthreads();
         if (threadIdx.x == 0) {
-            if constexpr (!multi) {
+            if constexpr (cluster) {
+                if (rank == 0) {  // the team's
+                    sm.mine[0] = sm.run[0];
+                    sm.mine[1] = sm.run[1];
+                }
+            } else if constexpr (!ring) {
                 // Iterations 0 .. it - 1 were counted when the next one began;
                 // the one the loop left by, or the last before a suspension:
                 const uint32_t last = status == kInf ? it - 1 : it;
@@ -1081,7 +1228,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         // Suspending: fold in what the iterations not tested yet found -- a
         // goal popped there is in no heap any more -- and stop on entries
         // they lost.
-        if constexpr (multi) {
+        if constexpr (ring) {
             if (threadIdx.x == 0) {
                 CutSlot* c = tm.ctl->cut + it % kCuts;
                 if (sm.agg.best != kInf) atomicMin(&c->best, sm.agg.best);
@@ -1106,6 +1253,12 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 best_r = uniform(sm.dec_best);
                 status = uniform(sm.dec_status);
             }
+        } else if constexpr (cluster) {
+            uint32_t pe = 0;  // raised by the last push of any block
+            if ((uint32_t)lane < tm.ctas)
+                pe = ld_cluster(&sm.slot[(it + kSlots - 1) % kSlots].claims, (uint32_t)lane).w;
+            if (it > 0 && __reduce_max_sync(kFull, pe) != 0) status = ST_HEAP_FULL;
+            cluster_sync();
         } else if (it > 0 && uniform(ld_vol(&sm.slot[(it + kSlots - 1) % kSlots].perr)) == ST_HEAP_FULL) {
             status = ST_HEAP_FULL;  // raised by the last push
         }
@@ -1127,10 +1280,6 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         __threadfence();
         ctl->life = LIFE_DONE;
     }
-    // The callers' next block barrier wants whole warps: this function is not
-    // inlined, and a lane that returned ahead of the leader's would reach it
-    // alone.
-    __syncwarp();
 }
 
 template <uint32_t KINDS, int MAXT, int TEAM>
@@ -1154,7 +1303,8 @@ __device__ __forceinline__ void dispatch(const LaunchParams& P, const TeamRef tm
 }
 
 // Persistent search kernel.
-//  * plain (team_ctas > 1): every block works on instance 0 (cooperative launch);
+//  * plain (team_ctas > 1): every block works on instance 0 (one cluster, or a
+//    cooperative launch);
 //  * batch/serve: blocks of the heavy teams first take heavy instances together
 //    (grids), then every block takes instances one block each from a work counter.
 // MAXT bounds the block size: 256 threads (8 warps) leave the compiler up to
@@ -1172,45 +1322,71 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(const __grid_constant__
             sm.slice = P.slice_iters;
         }
         __syncthreads();
-        if constexpr (plain) dispatch<KINDS, MAXT, TEAM_RING>(P, TeamRef{P.team_ctas, blockIdx.x, P.team, P.stage});
+        if constexpr (plain) {
+            const TeamRef tm{P.team_ctas, blockIdx.x, P.team, P.stage};
+            if constexpr (MAXT <= 256)
+                if (P.cluster) {
+                    dispatch<KINDS, MAXT, TEAM_CLUSTER>(P, tm);
+                    return;
+                }
+            dispatch<KINDS, MAXT, TEAM_RING>(P, tm);
+        }
         return;
     }
     if (many && P.n_heavy && blockIdx.x < P.heavy_teams * P.heavy_team) {
         const uint32_t t = blockIdx.x / P.heavy_team, rank = blockIdx.x % P.heavy_team;
-        TeamCtl* tc = P.heavy_ctl + t;
-        const TeamRef tm{P.heavy_team, rank, tc,
-                         reinterpret_cast<char*>(P.heavy_stage) + (size_t)t * P.heavy_stage_bytes};
-        for (;;) {
-            // Every block of the team is done with the previous instance here.
-            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
-            if (rank == 0 && threadIdx.x == 0) {
-                for (uint32_t k = 0; k < kCuts; ++k) {
-                    tc->cut[k].minf = kInf;
-                    tc->cut[k].claims = tc->cut[k].exps = 0;
-                    tc->cut[k].best = kInf;
-                    tc->cut[k].lossy = 0;
-                    tc->cut[k].err = 0;
-                    tc->cut[k].count = 0;
+        if (P.cluster) {
+            if constexpr (many) {
+                for (;;) {
+                    if (rank == 0 && threadIdx.x == 0) sm.inst = atomicAdd(P.heavy_next, 1u);
+                    cluster_sync();
+                    const uint32_t i = uniform(ld_cluster(&sm.inst, 0).x);
+                    cluster_sync();  // read by all before the first block's next use of it, or its exit
+                    if (i >= P.n_heavy) break;
+                    if (threadIdx.x == 0) {
+                        const uint32_t slot = P.heavy_order[i];
+                        sm.desc = P.insts[slot];
+                        sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
+                    }
+                    __syncthreads();
+                    dispatch<kind_bit(KIND_GRID), MAXT, TEAM_CLUSTER>(P, TeamRef{P.heavy_team, rank, nullptr, nullptr});
+                    __syncthreads();
                 }
-                tc->inst = atomicAdd(P.heavy_next, 1u);
             }
-            if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
-            const uint32_t i = ld_vol(&tc->inst);
-            if (i >= P.n_heavy) break;
-            if (threadIdx.x == 0) {
-                const uint32_t slot = P.heavy_order[i];
-                sm.desc = P.insts[slot];
-                sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
+        } else {
+            TeamCtl* tc = P.heavy_ctl + t;
+            const TeamRef tm{P.heavy_team, rank, tc,
+                             reinterpret_cast<char*>(P.heavy_stage) + (size_t)t * P.heavy_stage_bytes};
+            for (;;) {
+                // Every block of the team is done with the previous instance here.
+                if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
+                if (rank == 0 && threadIdx.x == 0) {
+                    for (uint32_t k = 0; k < kCuts; ++k) {
+                        tc->cut[k].minf = kInf;
+                        tc->cut[k].claims = tc->cut[k].exps = 0;
+                        tc->cut[k].best = kInf;
+                        tc->cut[k].lossy = 0;
+                        tc->cut[k].err = 0;
+                        tc->cut[k].count = 0;
+                    }
+                    tc->inst = atomicAdd(P.heavy_next, 1u);
+                }
+                if (!team_sync_grid(tc, P.heavy_team, P.barrier_timeout_ns)) break;
+                const uint32_t i = ld_vol(&tc->inst);
+                if (i >= P.n_heavy) break;
+                if (threadIdx.x == 0) {
+                    const uint32_t slot = P.heavy_order[i];
+                    sm.desc = P.insts[slot];
+                    sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
+                }
+                __syncthreads();
+                if constexpr (many) dispatch<kind_bit(KIND_GRID), MAXT, TEAM_RING>(P, tm);
             }
-            __syncthreads();
-            if constexpr (many) dispatch<kind_bit(KIND_GRID), MAXT, TEAM_RING>(P, tm);
-            __syncwarp();
         }
         __syncthreads();
     }
     for (;;) {
         if (threadIdx.x == 0) sm.inst = atomicAdd(P.next, 1u);
-        __syncwarp();
         __syncthreads();
         const uint32_t i = sm.inst;
         if (i >= P.n_insts) break;
@@ -1219,10 +1395,8 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(const __grid_constant__
             sm.desc = P.insts[slot];
             sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
         }
-        __syncwarp();
         __syncthreads();
         dispatch<KINDS, MAXT, TEAM_BLOCK>(P, TeamRef{1, 0, nullptr, nullptr});
-        __syncwarp();
         __syncthreads();
     }
 }

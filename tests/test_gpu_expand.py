@@ -47,3 +47,40 @@ def test_block_shapes_in_a_batch(engine, oracle, gastar, warps):
         b.rerun()
         assert [b.result(i, path=False).cost for i in range(len(b))] == cases
         b.close()
+
+
+@pytest.mark.parametrize("blocks,warps", [(2, 1), (2, 8), (3, 3), (7, 2), (15, 8), (16, 1), (16, 8), (17, 8)])
+def test_cluster_teams(engine, oracle, gastar, blocks, warps):
+    """Clusters of every size class (17 blocks: a ring team), heaps and
+    buckets, a budget that ends the search early, then a normal solve."""
+    for open_list in (0, 1):
+        kw = dict(expansion_width=4, warps_per_block=warps, num_queues=4 * warps * blocks, open_list=open_list)
+        for w, h, delta in ((5, 3, 0), (83, 64, 0), (83, 64, 12)):
+            wts = gastar.gen_grid(w, h, 140 + w, 0.2)
+            r = engine.solve_grid(wts, (0, 0), (w - 1, h - 1), delta=delta, **kw)
+            o, _ = oracle.grid_astar(wts, (0, 0), (w - 1, h - 1), path=False)
+            assert r.status_name == "OK" and r.cost == o.cost
+            assert oracle.grid_validate(wts, (0, 0), (w - 1, h - 1), r.path) == (True, r.cost)
+            assert r.expansions > 0 and r.generated >= r.pushes > 0
+        for n, walk in ((3, (24, 30)), (4, (20, 30)), (5, (12, 18))):
+            s, g = gastar.gen_sliding(n, 170 + n, *walk)
+            r = engine.solve_sliding(s, g, n, **kw)
+            o, _ = oracle.sliding_astar(n, s, g, path=False)
+            assert r.status_name == "OK" and r.cost == o.cost
+            assert oracle.sliding_validate(n, s, g, r.path) == (True, r.cost)
+        s, g = gastar.gen_sliding(4, 199, 60, 60)
+        r = engine.solve_sliding(s, g, 4, max_iterations=3, **kw)
+        assert r.status_name == "BUDGET" and r.iterations <= 6
+        wall = np.zeros((9, 9), dtype=np.uint8)
+        wall[0, 0] = wall[8, 8] = 1
+        assert engine.solve_grid(wall, (0, 0), (8, 8), **kw).status_name == "NO_PATH"
+
+
+def test_cluster_heap_overflow_is_regrown(engine, oracle, gastar):
+    """A heap that fills in a cluster team loses entries: without regrow the
+    status says so, with it the cost is right."""
+    wts = gastar.gen_grid(220, 180, 77, 0.1)
+    o, _ = oracle.grid_astar(wts, (0, 0), (219, 179), path=False)
+    kw = dict(expansion_width=1, warps_per_block=1, num_queues=2, heap_entries=1, heuristic=2)
+    r = engine.solve_grid(wts, (0, 0), (219, 179), **kw)
+    assert r.status_name == "OK" and r.cost == o.cost
