@@ -139,6 +139,7 @@ struct gastar_batch {
     std::vector<uint8_t> promotable;   // re-solved by the plain engine past the budget
     uint32_t n_heavy = 0, heavy_teams = 0;
     uint64_t heavy_stage_bytes = 0;
+    bool cluster = false;        // its teams are thread-block clusters
     uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap nodes per warp
     DevBuf team_ctl, team_stage;
     uint32_t promoted = 0;
@@ -376,6 +377,16 @@ int batch_upload(gastar_batch* b) {
             std::fill(b->heavy.begin(), b->heavy.end(), 0);
         }
     }
+    // Teams are clusters (a grid of whole clusters) where as many blocks are
+    // resident that way.
+    b->cluster = false;
+    if (b->n_heavy && cluster_team_size(T)) {
+        const uint32_t whole = (b->blocks + T - 1) / T;
+        if ((uint32_t)occupancy_clusters(kKindsAll, b->threads, b->smem, T) >= whole) {
+            b->cluster = true;
+            b->blocks = whole * T;
+        }
+    }
     std::vector<PartPlan> plans(n);
     std::vector<uint64_t> part_off(n);
     uint64_t arena_bytes = 0;
@@ -423,7 +434,7 @@ int batch_upload(gastar_batch* b) {
     std::stable_sort(horder.begin(), horder.end(), by_est);
     b->n_sched = (uint32_t)order.size();
     order.insert(order.end(), horder.begin(), horder.end());
-    if (b->n_heavy) {
+    if (b->n_heavy && !b->cluster) {
         b->heavy_stage_bytes = team_stage_bytes(T, pc.warps, pc.ew, 8, 16);
         if (!b->team_ctl.ensure(sizeof(TeamCtl) * b->heavy_teams) ||
             !b->team_stage.ensure(b->heavy_stage_bytes * b->heavy_teams))
@@ -471,10 +482,12 @@ int batch_enqueue(gastar_batch* b, cudaStream_t st, bool capturing) {
         P.heavy_team = b->cfg.heavy_team;
         P.heavy_teams = b->heavy_teams;
         P.heavy_next = reinterpret_cast<uint32_t*>(b->counters.p) + 4;
+        P.cluster = b->cluster ? 1u : 0u;
         P.heavy_ctl = reinterpret_cast<TeamCtl*>(b->team_ctl.p);
         P.heavy_stage = b->team_stage.p;
         P.heavy_stage_bytes = b->heavy_stage_bytes;
-        if (!cuda_ok(cudaMemsetAsync(b->team_ctl.p, 0, sizeof(TeamCtl) * b->heavy_teams, st), "cudaMemsetAsync"))
+        if (!b->cluster &&
+            !cuda_ok(cudaMemsetAsync(b->team_ctl.p, 0, sizeof(TeamCtl) * b->heavy_teams, st), "cudaMemsetAsync"))
             return GASTAR_CUDA_ERROR;
     }
     // Inside a graph capture, external records stay timing events.

@@ -53,6 +53,9 @@ int occupancy_blocks(struct ::gastar_ctx* c, uint32_t kinds, uint32_t threads, s
 // Clusters of `size` blocks of this shape that are resident at once (0: the
 // size or the shape does not fit).
 int occupancy_clusters(uint32_t kinds, uint32_t threads, size_t smem, uint32_t size);
+// Whether heavy teams of `size` blocks run as clusters: sizes that every GPC
+// can be cut into, up to the largest cluster.
+inline bool cluster_team_size(uint32_t size) { return size == 2 || size == 4 || size == 8 || size == 16; }
 int device_min_weight(struct ::gastar_ctx* c, const uint8_t* d_w, uint64_t cells, cudaStream_t st,
                       uint32_t* out);
 // Places a grid's weights from the caller's host buffer at d_dst and returns

@@ -103,6 +103,7 @@ struct gastar_server {
     RangeAlloc walloc;
     uint32_t heavy_teams = 0;   // team buffers allocated (the most teams a launch can hold)
     uint32_t resident = 0;      // blocks resident on the device at once
+    uint32_t clusters = 0;      // clusters of heavy_team blocks resident at once (0: no such clusters)
     uint64_t heavy_stage_bytes = 0;
     uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap nodes per warp
     RangeAlloc alloc;  // the arena
@@ -358,6 +359,8 @@ gastar_server* gastar_serve_create(gastar_ctx* c, const gastar_serve_config* cfg
         // uses as many as its heavy requests and the light ones leave room for.
         s->heavy_teams = cf.heavy_teams ? cf.heavy_teams : resident / cf.heavy_team;
         s->heavy_teams = std::min(s->heavy_teams, resident / cf.heavy_team);
+        if (cluster_team_size(cf.heavy_team))
+            s->clusters = (uint32_t)occupancy_clusters(kKindsAll, s->threads, s->smem, cf.heavy_team);
         s->heavy_stage_bytes = team_stage_bytes(cf.heavy_team, cf.warps_per_block, cf.expansion_width, 8, 16);
         if (!s->heavy_teams || !s->team_ctl.ensure(sizeof(TeamCtl) * s->heavy_teams) ||
             !s->team_stage.ensure(s->heavy_stage_bytes * s->heavy_teams))
@@ -536,6 +539,16 @@ int gastar_serve_step(gastar_server* s) {
         const uint32_t T = s->cfg.heavy_team;
         const uint32_t teams = std::min(team_cap, (uint32_t)heavy.size());
         blocks = std::min(s->resident, teams * T + (uint32_t)light.size());
+        // Teams are clusters while the launch's blocks are all resident that
+        // way (a GPC's SMs are not a multiple of eight: fewer eight-block
+        // clusters fit than teams).  Eight 2048^2 grids: 37.5 against 45.9 ms
+        // of search kernels; sixteen of 1200^2, of which only some fit: 34.4
+        // against 23.2, hence the ring then.  A request's saved state is the
+        // same either way.
+        if (s->clusters && (blocks + T - 1) / T <= s->clusters) {
+            blocks = (blocks + T - 1) / T * T;
+            P.cluster = 1;
+        }
         P.heavy_order = reinterpret_cast<const uint32_t*>(s->order.p) + light.size();
         // At most heavy_set x teams heavy requests, the largest first, take
         // turns in a launch: fewer grids per launch keep their frontiers in
@@ -551,7 +564,8 @@ int gastar_serve_step(gastar_server* s) {
         P.heavy_ctl = reinterpret_cast<TeamCtl*>(s->team_ctl.p);
         P.heavy_stage = s->team_stage.p;
         P.heavy_stage_bytes = s->heavy_stage_bytes;
-        if (!cuda_ok(cudaMemsetAsync(s->team_ctl.p, 0, sizeof(TeamCtl) * teams, st), "cudaMemsetAsync"))
+        if (!P.cluster &&
+            !cuda_ok(cudaMemsetAsync(s->team_ctl.p, 0, sizeof(TeamCtl) * teams, st), "cudaMemsetAsync"))
             return GASTAR_CUDA_ERROR;
     }
     cudaEventRecord(s->e0, st);
