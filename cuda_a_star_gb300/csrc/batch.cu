@@ -132,7 +132,7 @@ struct gastar_batch {
     // Grid weights, copied to the device when the grid is added: bump
     // allocation in chunks of at least 256 MiB, freed with the batch.
     // Re-run batches and autotuner trials point at their parent's copies.
-    std::vector<void*> grid_chunks;
+    std::vector<DevBuf> grid_chunks;
     size_t grid_chunk_used = 0, grid_chunk_cap = 0;
     uint64_t grid_bytes = 0, grid_h2d = 0;
     std::vector<uint8_t> heavy;        // solved by a multi-block team
@@ -171,17 +171,21 @@ uint8_t* grid_alloc(gastar_batch* b, size_t bytes) {
     bytes = (bytes + 255) & ~(size_t)255;
     if (b->grid_chunks.empty() || b->grid_chunk_used + bytes > b->grid_chunk_cap) {
         const size_t cap = std::max<size_t>(bytes, (size_t)256 << 20);
-        void* c = nullptr;
-        if (cudaMalloc(&c, cap) != cudaSuccess) {
+        DevBuf c;
+        if (!b->ctx->spare.take(c, cap, SPARE_GRIDS) && !c.ensure(cap)) {
+            b->ctx->spare.drop();
             cudaGetLastError();
-            return nullptr;
+            if (!c.ensure(cap)) {
+                cudaGetLastError();
+                return nullptr;
+            }
         }
         b->grid_chunks.push_back(c);
-        b->grid_chunk_cap = cap;
+        b->grid_chunk_cap = c.n;
         b->grid_chunk_used = 0;
-        b->grid_bytes += cap;
+        b->grid_bytes += c.n;
     }
-    uint8_t* r = static_cast<uint8_t*>(b->grid_chunks.back()) + b->grid_chunk_used;
+    uint8_t* r = static_cast<uint8_t*>(b->grid_chunks.back().p) + b->grid_chunk_used;
     b->grid_chunk_used += bytes;
     return r;
 }
@@ -230,8 +234,9 @@ void gastar_batch_destroy(gastar_batch* b) {
     cudaStreamSynchronize(b->ctx->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     gastar_batch_destroy(b->sub);
-    b->arena.release();
-    for (void* c : b->grid_chunks) cudaFree(c);
+    // The stream is idle: the next batch of this context may have the memory.
+    b->ctx->spare.give(b->arena, SPARE_ARENA);
+    for (DevBuf& c : b->grid_chunks) b->ctx->spare.give(c, SPARE_GRIDS);
     b->descs.release();
     b->ctls.release();
     b->order.release();
@@ -397,11 +402,17 @@ int batch_upload(gastar_batch* b) {
         arena_bytes += plans[i].bytes;
         b->path_words += plans[i].path_words;
     }
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    if (arena_bytes + (64ull << 20) > free_b) {
-        set_error("batch partitions exceed free device memory");
-        return GASTAR_OUT_OF_MEMORY;
+    if (!c->spare.take(b->arena, arena_bytes, SPARE_ARENA)) {
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        if (arena_bytes + (64ull << 20) > free_b) {
+            c->spare.drop();
+            cudaMemGetInfo(&free_b, &total_b);
+        }
+        if (arena_bytes + (64ull << 20) > free_b) {
+            set_error("batch partitions exceed free device memory");
+            return GASTAR_OUT_OF_MEMORY;
+        }
     }
     if (!b->arena.ensure(arena_bytes) || !b->descs.ensure(sizeof(InstDesc) * n) || !b->ctls.ensure(sizeof(InstCtl) * (n + 1)) ||
         !b->order.ensure(sizeof(uint32_t) * n) || !b->counters.ensure(64) ||

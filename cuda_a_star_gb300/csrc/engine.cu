@@ -73,6 +73,33 @@ bool DevBuf::ensure(size_t bytes) {
     return true;
 }
 
+bool SpareMemory::take(DevBuf& b, size_t bytes, int which) {
+    std::lock_guard<std::mutex> lk(mu_);
+    DevBuf& k = kept_[which];
+    if (!k.p || k.n < bytes) return false;
+    b = k;
+    b.fresh = true;
+    k = DevBuf();
+    return true;
+}
+
+void SpareMemory::give(DevBuf& b, int which) {
+    std::lock_guard<std::mutex> lk(mu_);
+    DevBuf& k = kept_[which];
+    if (b.p && b.n <= kSpareMax && b.n > k.n) std::swap(b, k);
+    b.release();
+}
+
+bool SpareMemory::drop() {
+    std::lock_guard<std::mutex> lk(mu_);
+    bool any = false;
+    for (DevBuf& k : kept_) {
+        any = any || k.p;
+        k.release();
+    }
+    return any;
+}
+
 const void* search_kernel_for(uint32_t kinds, uint32_t threads) {
     if (threads > 256) return search_kernel_all16();  // 9..16 warps: all kinds
     switch (kinds) {
@@ -363,6 +390,7 @@ void gastar_destroy(gastar_ctx* c) {
     c->path.release();
     c->misc.release();
     c->weights.release();
+    c->spare.drop();
     destroy_stager(c->stager);
     if (c->h_ctl) cudaFreeHost(c->h_ctl);
     if (c->h_launch) cudaFreeHost(c->h_launch);
@@ -713,6 +741,10 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
     for (;;) {
         ++attempts;
         int rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
+        if (rc == GASTAR_OUT_OF_MEMORY && c->spare.drop()) {  // again without what was kept for batches
+            cudaGetLastError();
+            rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
+        }
         if (rc != GASTAR_OK) return rc;
         if (!cfg.regrow) break;
         if (ctl.status == ST_TABLE_FULL && pp.kind != KIND_GRID && table_log2 < max_log2) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -19,6 +20,28 @@ struct DevBuf {
     bool ensure(size_t bytes);  // grows (contents are not kept)
     void release();
 };
+
+// Device memory of a destroyed batch, kept by its context for the next one:
+// mapping and unmapping a batch's partitions (11 GB for 512 8-puzzles) takes
+// longer than searching them.  One partition arena and one chunk of grid
+// weights, at most kSpareMax bytes each; whatever else of this library finds
+// too little memory on the device takes them back first (drop), and the
+// context's end releases them.
+class SpareMemory {
+public:
+    static constexpr size_t kSpareMax = (size_t)16 << 30;
+    // Moves a kept buffer of at least `bytes` into `b` (empty); false: none.
+    bool take(DevBuf& b, size_t bytes, int which);
+    // Keeps `b`, or what was kept if that is larger, and releases the other.
+    void give(DevBuf& b, int which);
+    // Releases what is kept; false: nothing was.
+    bool drop();
+
+private:
+    std::mutex mu_;
+    DevBuf kept_[2];
+};
+enum { SPARE_ARENA = 0, SPARE_GRIDS = 1 };
 
 void set_error(const std::string& s);
 bool cuda_ok(cudaError_t e, const char* what);
@@ -115,6 +138,7 @@ struct gastar_ctx {
     bool can_read_host = false;    // kernels read pageable host memory through the host's
                                    // page tables (ATS over NVLink-C2C on Grace)
     int upload_mode = 2;           // grid uploads: 0 copy, 1 read in place, 2 staged
+    gastar::SpareMemory spare;
     gastar::HostStager* stager = nullptr;  // staged uploads (pinned ring, host threads)
     bool table_dirty = true;       // hash table needs a full clear before the next solve
     uint32_t prev_slot_words = 2;  // slot width of the solve that filled the touched list

@@ -329,6 +329,7 @@ gastar_server* gastar_serve_create(gastar_ctx* c, const gastar_serve_config* cfg
     cf.expansion_width = std::min(32u, cf.expansion_width);
     if (cf.load_factor <= 0.f) cf.load_factor = 0.75f;
     if (!cf.slice_iters) cf.slice_iters = 128;
+    c->spare.drop();  // the budget is a share of the memory that is free
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     uint64_t budget = cf.budget_bytes ? cf.budget_bytes : (120ull << 30);
