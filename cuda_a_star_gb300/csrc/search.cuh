@@ -325,7 +325,7 @@ struct CtaShared {
     unsigned long long base[2];  // claims, expansions before this launch
     unsigned long long wcnt[kMaxWarps][3];  // per warp: stale, generated, pushed in this launch
     unsigned long long t_start;  // search start on the device clock
-    uint32_t dec_status, dec_best, dec_fmin, push_count;  // thread 0 -> block
+    uint32_t dec_status, dec_best, dec_fmin, push_count, push_ok;  // ring teams: its two threads -> block
     // Cluster teams, warp 0 -> block: best, error, least open f, chunks in
     // all, entries per chunk; per block the chunks before its own, its entries.
     uint32_t plan[8], plan_before[kMaxClusterBlocks], plan_count[kMaxClusterBlocks];
@@ -952,17 +952,18 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             // ---- one hand-off per iteration: publish cut `it` and this
             // block's stage region, then wait for the region this block
             // pushes and test cut it - kCutLag (a_star.h:260-262) ----
+            // Thread 0 publishes and waits for the region; meanwhile the second
+            // warp's first thread waits for the cut and tests it (one after
+            // the other they took 1.5-3.6 k cycles more of an iteration).
             __syncthreads();  // every warp's stage writes and counters are done
             if (threadIdx.x == 0) {
                 CutSlot* cuts = tm.ctl->cut;
                 unsigned long long* const rw = ready + (size_t)(it % kStageRing) * tm.ctas;
                 const uint32_t from = (rank + it) % tm.ctas;
-                // Both awaited words are read first, relaxed (the fence below
-                // orders them before what follows): their round trips overlap
+                // The awaited word is read first, relaxed (the fence below
+                // orders it before what follows): its round trip overlaps
                 // this block's publication.
                 unsigned long long wfrom = from == rank ? 0ull : ld_relaxed_u64(rw + from);
-                const CutSlot* t = cuts + (it + kCuts - kCutLag) % kCuts;
-                const uint32_t tseen = it >= kCutLag ? ld_relaxed_u32(&t->count) : 0u;
                 const uint32_t lossy = sm.agg.err ? sm.agg.err : sm.agg_err_prev;
                 uint32_t err = 0;
                 if (leader) {
@@ -982,18 +983,20 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 CutSlot* c = cuts + it % kCuts;
                 const uint32_t cm = sm.agg_minheap < sm.agg.minstage ? sm.agg_minheap : sm.agg.minstage;
                 if (cm != kInf) atomicMin(&c->minf, cm);
-                if (sm.agg.claims) atomicAdd(&c->claims, (unsigned long long)sm.agg.claims);
-                if (sm.agg.exps) atomicAdd(&c->exps, (unsigned long long)sm.agg.exps);
+                // The team's counts are for its budgets only.
+                if (sm.agg.claims && d.table_limit != ~0ull)
+                    atomicAdd(&c->claims, (unsigned long long)sm.agg.claims);
+                if (sm.agg.exps && d.max_exp) atomicAdd(&c->exps, (unsigned long long)sm.agg.exps);
                 sm.mine[0] += sm.agg.claims;
                 sm.mine[1] += sm.agg.exps;
                 if (sm.agg.best != kInf) atomicMin(&c->best, sm.agg.best);
                 if (lossy) atomicCAS(&c->lossy, 0u, lossy);
                 if (err) atomicCAS(&c->err, 0u, err);
                 const uint32_t mine = sm.agg.count;
-                // One fence for both arrivals and both early reads: every
+                // One fence for both arrivals and the early read: every
                 // warp's stage writes (ordered before thread 0 by the block
                 // barrier) and the cut's updates precede the ready word and
-                // the cut arrival (release); the words read above precede
+                // the cut arrival (release); the word read above precedes
                 // everything after (acquire).
                 fence_acq_rel_gpu();
                 st_relaxed_u64(rw + rank, ((unsigned long long)(it + 1) << 32) | mine);
@@ -1001,24 +1004,30 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 slot_clear(sm.agg);
                 sm.agg_minheap = kInf;
                 sm.agg_err_prev = 0;
-                uint32_t dec = kInf, n = 0, dbest = kInf, dfmin = kInf;
+                uint32_t n = 0, got = 1;
                 if (from == rank)
                     n = mine;
                 else if (!team_wait_ready(rw + from, it + 1, wfrom, tm.ctl, P.barrier_timeout_ns))
-                    dec = ST_BARRIER;
+                    got = 0;
                 else
                     n = (uint32_t)wfrom;
-                if (dec == kInf && it >= kCutLag) {
+                sm.push_count = n;
+                sm.push_ok = got;
+            }
+            if (threadIdx.x == (W > 1 ? 32u : 0u)) {
+                uint32_t dec = kInf, dbest = kInf, dfmin = kInf;
+                if (it >= kCutLag) {
                     // Waits only while a block is more than kCutLag iterations behind.
-                    if (!team_wait_u32(&t->count, tm.ctas, tseen, tm.ctl, P.barrier_timeout_ns)) {
+                    const CutSlot* t = tm.ctl->cut + (it + kCuts - kCutLag) % kCuts;
+                    if (!team_wait_u32(&t->count, tm.ctas, ld_acquire_u32(&t->count), tm.ctl, P.barrier_timeout_ns)) {
                         dec = ST_BARRIER;
                     } else {
                         const uint32_t open_f = ld_vol(&t->minf);
                         dbest = ld_vol(&t->best);
                         uint32_t tl = ld_vol(&t->lossy), te = ld_vol(&t->err);
                         // Budgets from the team's totals, the same in every block.
-                        sm.run[0] += ld_vol64(&t->claims);
-                        sm.run[1] += ld_vol64(&t->exps);
+                        if (d.table_limit != ~0ull) sm.run[0] += ld_vol64(&t->claims);
+                        if (d.max_exp) sm.run[1] += ld_vol64(&t->exps);
                         if (!tl && sm.base[0] + sm.run[0] > d.table_limit) tl = ST_TABLE_FULL;
                         if (!te && d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) te = ST_BUDGET;
                         const uint32_t bb = dbest < best_r ? dbest : best_r;
@@ -1032,14 +1041,13 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 sm.dec_status = dec;
                 sm.dec_best = dbest;
                 sm.dec_fmin = dfmin;
-                sm.push_count = n;
             }
             __syncthreads();
             {
                 const uint32_t db = uniform(sm.dec_best), df = uniform(sm.dec_fmin);
                 best_r = db < best_r ? db : best_r;
                 if (df != kInf) fmin = df;
-                status = uniform(sm.dec_status);
+                status = uniform(sm.push_ok) ? uniform(sm.dec_status) : (uint32_t)ST_BARRIER;
             }
             if (status != kInf) break;
         } else {
