@@ -545,6 +545,10 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
     // Rounds whose probes are in flight together.  Blocks of 9 to 16 warps
     // have 128 registers per thread and overlap their warps' rounds instead.
     constexpr int RB = MAXT > 256 ? 1 : KW == 1 ? 4 : 2;
+    // The 16-warp kernel has 128 registers a thread and mostly pops 32 at
+    // once; the second way to pop cost its grids 100 bytes more of spilled
+    // registers (152 grids of 1000 x 1000 one block each: 39 -> 43 ms).
+    constexpr bool kFewPath = MAXT <= 256;
     CtaShared& sm = cta();
     const InstDesc& d = sm.desc;
     typename D::Ctx& ctx = shared_ctx<D>();
@@ -644,7 +648,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         best_r = uniform_if(D::is_goal(ctx, ctx.start)) ? 0u : kInf;
         have_prev = true;  // the start is the only open entry; every slot starts empty
     } else {
-        heap_restore(hp, d.heap_hdr + 2 * hid, lane);
+        heap_restore<kFewPath>(hp, d.heap_hdr + 2 * hid, lane);
         bq_restore(bq, bq_words() + 2 * (size_t)d.heaps * bq.P + (size_t)hid * kBucketStateWords, lane);
         best_r = uniform(ld_vol(&ctl->best));
         have_prev = false;
@@ -728,7 +732,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                                  : kInfPrio;
         E e;
         const uint32_t cnt =
-            open_pop(hp, bq, uniform(d.wide_after && it0 + it >= d.wide_after ? d.ew_wide : d.ew), lim, e, lane);
+            open_pop<kFewPath>(hp, bq, uniform(d.wide_after && it0 + it >= d.wide_after ? d.ew_wide : d.ew), lim, e, lane);
         bool act = (uint32_t)lane < cnt;
         const KeyT k = D::key_of(e);
         const uint32_t g = prio_g(e.prio);
