@@ -28,13 +28,15 @@ inline __host__ __device__ size_t stage_entries_per_buffer(uint32_t heaps, uint3
 
 // Multi-block teams run their iterations without a team barrier.  Block b
 // stages its successors of iteration i into region b of stage buffer
-// i % kStageRing; after its expansion it publishes, behind one release fence,
-// ready[b] = i + 1 and its part of cut i (heap minimum after the previous
-// push, minimum of what it staged, goals, errors, counts).  Block c then
+// i % kStageRing; after its expansion it publishes, each behind a release
+// fence, ready[b] = i + 1 and its part of cut i (heap minimum after the
+// previous push, minimum of what it staged, goals, errors, counts).  Block c then
 // pushes the region of block (c + i) % blocks once that block is ready.  Cut
 // i is tested at iteration i + kCutLag, so no block runs more than kCutLag
 // iterations ahead of another, and a stage buffer is always consumed before
 // it is written again.
+// A lag of 3 gained no block anything (grids 0.1-0.6 % slower, 24-puzzles
+// 2.9 %): blocks wait for the slowest of their partners, not for the cut.
 constexpr uint32_t kStageRing = 4;
 constexpr uint32_t kCutLag = 2;
 constexpr uint32_t kCuts = 16;  // cut slots in the ring (> 3 * kCutLag + 2)

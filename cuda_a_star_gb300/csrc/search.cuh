@@ -956,21 +956,36 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             // ---- one hand-off per iteration: publish cut `it` and this
             // block's stage region, then wait for the region this block
             // pushes and test cut it - kCutLag (a_star.h:260-262) ----
-            // Thread 0 publishes and waits for the region; meanwhile the second
-            // warp's first thread waits for the cut and tests it (one after
-            // the other they took 1.5-3.6 k cycles more of an iteration).
+            // Thread 0 publishes the region and waits for the one it takes;
+            // the second warp's first thread (of a one-warp block, thread 0
+            // in between) does the same for the cuts.  A chain of round trips
+            // to L2 (fence 1.0 k cycles, store to load 1.4 k or more), so the
+            // region, which the push waits for, goes first and by itself (behind the cut's
+            // updates: grid 1021^2 6.11 ms, so: 5.91).
             __syncthreads();  // every warp's stage writes and counters are done
+            const uint32_t cut_thread = W > 1 ? 32u : 0u;
+            unsigned long long* const rw = ready + (size_t)(it % kStageRing) * tm.ctas;
+            unsigned long long wfrom = 0;
+            uint32_t from = 0, mine = 0;
             if (threadIdx.x == 0) {
+                from = (rank + it) % tm.ctas;
+                // The awaited word is read first, relaxed; its round trip
+                // overlaps the fence, which orders it before what follows
+                // (acquire) and every warp's stage writes, ordered before
+                // thread 0 by the block barrier, before the ready word (release).
+                wfrom = ld_relaxed_u64(rw + from);
+                mine = sm.agg.count;
+                sm.agg.count = 0;
+                fence_acq_rel_gpu();
+                st_relaxed_u64(rw + rank, ((unsigned long long)(it + 1) << 32) | mine);
+            }
+            if (threadIdx.x == cut_thread) {
                 CutSlot* cuts = tm.ctl->cut;
-                unsigned long long* const rw = ready + (size_t)(it % kStageRing) * tm.ctas;
-                const uint32_t from = (rank + it) % tm.ctas;
-                // The awaited word is read first, relaxed (the fence below
-                // orders it before what follows): its round trip overlaps
-                // this block's publication.
-                unsigned long long wfrom = from == rank ? 0ull : ld_relaxed_u64(rw + from);
+                const CutSlot* t = cuts + (it + kCuts - kCutLag) % kCuts;
+                const uint32_t tseen = it >= kCutLag ? ld_relaxed_u32(&t->count) : 0u;
                 const uint32_t lossy = sm.agg.err ? sm.agg.err : sm.agg_err_prev;
                 uint32_t err = 0;
-                if (leader) {
+                if (rank == 0) {
                     if (it >= 2 * kCutLag + 2) {  // every block has read it; none writes it yet
                         CutSlot* r = cuts + (it - 2 * kCutLag - 2) % kCuts;
                         r->minf = kInf;
@@ -996,34 +1011,19 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 if (sm.agg.best != kInf) atomicMin(&c->best, sm.agg.best);
                 if (lossy) atomicCAS(&c->lossy, 0u, lossy);
                 if (err) atomicCAS(&c->err, 0u, err);
-                const uint32_t mine = sm.agg.count;
-                // One fence for both arrivals and the early read: every
-                // warp's stage writes (ordered before thread 0 by the block
-                // barrier) and the cut's updates precede the ready word and
-                // the cut arrival (release); the word read above precedes
-                // everything after (acquire).
+                // The cut's updates, and every warp's reads of the last
+                // region, precede the arrival (release); the early read
+                // precedes everything after (acquire).
                 fence_acq_rel_gpu();
-                st_relaxed_u64(rw + rank, ((unsigned long long)(it + 1) << 32) | mine);
                 red_relaxed_add_u32(&c->count, 1u);
-                slot_clear(sm.agg);
+                sm.agg.err = sm.agg.claims = sm.agg.exps = sm.agg.perr = 0;  // not the count
+                sm.agg.minstage = sm.agg.best = sm.agg.minheap = kInf;
                 sm.agg_minheap = kInf;
                 sm.agg_err_prev = 0;
-                uint32_t n = 0, got = 1;
-                if (from == rank)
-                    n = mine;
-                else if (!team_wait_ready(rw + from, it + 1, wfrom, tm.ctl, P.barrier_timeout_ns))
-                    got = 0;
-                else
-                    n = (uint32_t)wfrom;
-                sm.push_count = n;
-                sm.push_ok = got;
-            }
-            if (threadIdx.x == (W > 1 ? 32u : 0u)) {
                 uint32_t dec = kInf, dbest = kInf, dfmin = kInf;
                 if (it >= kCutLag) {
                     // Waits only while a block is more than kCutLag iterations behind.
-                    const CutSlot* t = tm.ctl->cut + (it + kCuts - kCutLag) % kCuts;
-                    if (!team_wait_u32(&t->count, tm.ctas, ld_acquire_u32(&t->count), tm.ctl, P.barrier_timeout_ns)) {
+                    if (!team_wait_u32(&t->count, tm.ctas, tseen, tm.ctl, P.barrier_timeout_ns)) {
                         dec = ST_BARRIER;
                     } else {
                         const uint32_t open_f = ld_vol(&t->minf);
@@ -1045,6 +1045,15 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 sm.dec_status = dec;
                 sm.dec_best = dbest;
                 sm.dec_fmin = dfmin;
+            }
+            if (threadIdx.x == 0) {
+                uint32_t got = 1;
+                if (from == rank)
+                    wfrom = mine;
+                else if (!team_wait_ready(rw + from, it + 1, wfrom, tm.ctl, P.barrier_timeout_ns))
+                    got = 0;
+                sm.push_count = (uint32_t)wfrom;
+                sm.push_ok = got;
             }
             __syncthreads();
             {
