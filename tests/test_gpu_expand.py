@@ -84,3 +84,29 @@ def test_cluster_heap_overflow_is_regrown(engine, oracle, gastar):
     kw = dict(expansion_width=1, warps_per_block=1, num_queues=2, heap_entries=1, heuristic=2)
     r = engine.solve_grid(wts, (0, 0), (219, 179), **kw)
     assert r.status_name == "OK" and r.cost == o.cost
+
+
+@pytest.mark.parametrize("team", [2, 3, 4, 8, 16, 17])
+@pytest.mark.parametrize("instances", [2, 150])
+def test_heavy_teams(engine, oracle, gastar, team, instances):
+    """Heavy grids solved by clusters, or by ring teams where the clusters of
+    all teams are not resident at once (many instances) or the size is not a
+    cluster's (17): one launch of a batch, and a server whose searches are
+    suspended every few iterations with part of their roots popped."""
+    sides = [40 + (7 * i) % 23 for i in range(instances)]
+    grids = [gastar.gen_grid(s, s + 2, 300 + i, 0.2) for i, s in enumerate(sides)]
+    want = [oracle.grid_astar(w, (0, 0), (s - 1, s + 1), path=False)[0].cost for w, s in zip(grids, sides)]
+    kw = dict(warps_per_block=2, expansion_width=3, heavy_team=team, heavy_cells=1000)
+    b = engine.batch(**kw)
+    for w, s in zip(grids, sides):
+        b.add_grid(w, (0, 0), (s - 1, s + 1))
+    b.run()
+    assert [b.result(i, path=False).cost for i in range(instances)] == want
+    b.close()
+    srv = engine.server(slice_iters=16, budget_bytes=4 << 30, heavy_teams=min(instances, 8), **kw)
+    ids = [srv.submit_grid(w, (0, 0), (s - 1, s + 1)) for w, s in zip(grids, sides)]
+    got = srv.drain(ids)
+    srv.close()
+    assert [got[i].cost for i in ids] == want
+    for i, w, s in zip(ids, grids, sides):
+        assert oracle.grid_validate(w, (0, 0), (s - 1, s + 1), got[i].path) == (True, got[i].cost)
