@@ -543,8 +543,12 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
     constexpr int LPE = lanes_per_entry(MAXN);  // lanes per entry: one per move
     constexpr int EPR = 32 / LPE;               // entries per expansion round
     // Rounds whose probes are in flight together.  Blocks of 9 to 16 warps
-    // have 128 registers per thread and overlap their warps' rounds instead.
-    constexpr int RB = MAXT > 256 ? 1 : KW == 1 ? 4 : 2;
+    // have 128 registers per thread: their grids take two rounds (152 grids of
+    // 1000 x 1000, one block each: 28.9 -> 24.1 ms, with four 24.6), as far as
+    // no register spills (with 120 bytes of spills two rounds took 34 ms);
+    // their boards, bound by claims in cold tables, lose by it (15-puzzles
+    // 21.7 -> 23.2 us an iteration).
+    constexpr int RB = MAXT > 256 ? (D::kDense ? 2 : 1) : KW == 1 ? 4 : 2;
     // The 16-warp kernel has 128 registers a thread and mostly pops 32 at
     // once; the second way to pop cost its grids 100 bytes more of spilled
     // registers (152 grids of 1000 x 1000 one block each: 39 -> 43 ms).
@@ -1323,6 +1327,25 @@ __device__ __forceinline__ void dispatch(const LaunchParams& P, const TeamRef tm
     }
 }
 
+// The block's next instance into its shared state; false: none is left.  A
+// function of its own so that nothing of it, hoisted out of the caller's loop,
+// holds registers across a search: the 16-warp kernel's searches spilled 120
+// bytes for grids and 132 for boards with it in the loop, 8 and 44 without.
+inline __device__ __noinline__ bool take_instance(const LaunchParams& P) {
+    CtaShared& sm = cta();
+    if (threadIdx.x == 0) sm.inst = atomicAdd(P.next, 1u);
+    __syncthreads();
+    const uint32_t i = sm.inst;
+    if (i >= P.n_insts) return false;
+    if (threadIdx.x == 0) {
+        const uint32_t slot = P.order ? P.order[i] : i;
+        sm.desc = P.insts[slot];
+        sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
+    }
+    __syncthreads();
+    return true;
+}
+
 // Persistent search kernel.
 //  * plain (team_ctas > 1): every block works on instance 0 (one cluster, or a
 //    cooperative launch);
@@ -1406,17 +1429,7 @@ __global__ void __launch_bounds__(MAXT, 1) search_kernel(const __grid_constant__
         }
         __syncthreads();
     }
-    for (;;) {
-        if (threadIdx.x == 0) sm.inst = atomicAdd(P.next, 1u);
-        __syncthreads();
-        const uint32_t i = sm.inst;
-        if (i >= P.n_insts) break;
-        if (threadIdx.x == 0) {
-            const uint32_t slot = P.order ? P.order[i] : i;
-            sm.desc = P.insts[slot];
-            sm.slice = P.slices ? P.slices[slot] : P.slice_iters;
-        }
-        __syncthreads();
+    while (take_instance(P)) {
         dispatch<KINDS, MAXT, TEAM_BLOCK>(P, TeamRef{1, 0, nullptr, nullptr});
         __syncthreads();
     }
