@@ -443,11 +443,11 @@ struct PlainShape {
 // Shape of a ring team with the automatic widths: eight warps on every SM,
 // popping few entries each.  An iteration lasts as long as its slowest warp,
 // and a warp expands its pops in rounds (four grid cells, eight boards), so
-// many warps with one or two rounds beat fewer with more.  Measured: 16
-// 15-puzzles at Q = 16384 12.6 ms with 16-wide pops on 128 blocks, 10.5 with
-// 8-wide on 152 (4-wide: 13.0, too few pops); 1021^2 grid 11.3 ms with 16,
-// 9.2 with 8, 8.1 with 4; 4096^2 grid 49.5, 39.5 and 43.7 -- its frontier
-// (~4000 cells) fills 4-wide pops, hence the line at 2^22 cells.
+// many warps with one or two rounds beat fewer with more.  Measured on 152
+// blocks with 16-, 8- and 4-wide pops: 16 15-puzzles 10.6, 8.5 and 9.8 ms
+// (4-wide: too few pops); 1021^2 grid 8.8, 6.9 and 6.2 ms; 4096^2 grid 37.3,
+// 30.6 and 32.8 -- its frontier (~4000 cells) fills 4-wide pops, hence the
+// line at 2^22 cells.
 // Q above 16384 asks for throughput on hard puzzles: pops as wide as it says.
 static PlainShape ring_shape(const gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
     PlainShape s;
@@ -467,8 +467,9 @@ static PlainShape ring_shape(const gastar_ctx* c, const PlainProblem& pp, const 
 // memory behind one cluster barrier (~400 cycles) instead of the ring's
 // fences and flags (~2400), but have a tenth of the SMs: taken for searches
 // whose iterations hold a few hundred entries -- Q that small, 8-puzzles
-// (181,440 states in all; 0.175 against 0.225 ms) and grids up to 2^17 cells
-// (200 x 150: 1.18 against 1.44 ms; 517 x 389: 3.94 against 3.66 ms).
+// (181,440 states in all; 0.167 against 0.196 ms) and grids up to 2^17 cells
+// (200 x 150: 0.92 against 1.12 ms; 360 x 360: 2.18 against 2.13; 517 x 389:
+// 3.03 against 2.81).
 static PlainShape cluster_shape(const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
     PlainShape s;
     const bool fixed = cfg.expansion_width || cfg.warps_per_block;
@@ -509,8 +510,8 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     // iteration set rather than its depth; from then on every warp-heap pops
     // four times as many (at most 32).  On the 64 15-puzzles of the plain
     // benchmark (Q = 16384, 8-wide pops) the hardest took 333 iterations with
-    // twice the pops and takes 206 with four times; the 64 together 52.2 ->
-    // 50.3 ms.
+    // twice the pops and takes 206 with four times; the 64 together 4 % less
+    // time.
     const uint32_t ew_wide =
         multi && pp.kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 4 * ew) : ew;
     size_t smem = block_smem_bytes(kinds, W, ew, multi);

@@ -54,17 +54,18 @@ enum gastar_moves {
 
 /* Search parameters.  Zero fields take defaults (gastar_config_default). */
 typedef struct gastar_config {
-    uint32_t num_queues;       /* parallel pops per iteration (reference Q, main.cu:18) */
+    uint32_t num_queues;       /* parallel pops per iteration (reference Q, main.cu:18);
+                                  with automatic widths, an upper bound */
     uint32_t heuristic;        /* gastar_heuristic */
     uint32_t moves;            /* gastar_moves (sliding puzzles only) */
     uint32_t expansion_width;  /* entries each warp-heap pops per iteration, 1..32;
-                                  0 = auto, clamp(num_queues / 1024, 8, 32), and a
-                                  puzzle search on several blocks that passes 64
-                                  iterations then pops twice as many (at most 32) */
+                                  0 = auto, 4 to 8 on up to eight warps per SM
+                                  (puzzles above 16384 queues: up to 32), and a
+                                  puzzle search on many blocks that passes 64
+                                  iterations then pops four times as many (at most 32) */
     uint32_t warps_per_block;  /* warp-heaps per thread block, 1..16 (above 8: the
                                   512-thread kernel, at most 128 registers per thread);
-                                  0 = auto (8 when the blocks still cover half of the
-                                  SMs, else 4) */
+                                  0 = auto (8) */
     uint32_t max_blocks;       /* cap on thread blocks for one instance (0 = all SMs) */
     float load_factor;         /* table load limit before GASTAR_TABLE_FULL (0.5..0.9) */
     uint32_t table_log2;       /* hash-table slots = 2^table_log2 (0 = adaptive) */
