@@ -493,6 +493,12 @@ static PlainShape cluster_shape(const PlainProblem& pp, const gastar_config& cfg
     return s;
 }
 
+// A search whose table fills starts again in one of 2^kRegrowLog2 times the
+// slots.  64 15-puzzles (walk 20-80, Q = 4096), three of which fill the first
+// table, take 105 ms with doubling (up to four searches), 80.5 with 2, 60.8
+// with 3, 58.7 with 4, which may take twice the memory for that.
+constexpr uint32_t kRegrowLog2 = 3;
+
 // Runs the search (+ path rebuild) once with the given capacities.
 static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg,
                          uint32_t table_log2, uint64_t heap_entries, std::vector<uint64_t>* path_keys,
@@ -739,6 +745,7 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
     InstCtl ctl;
     AttemptStats as;
     uint32_t attempts = 0;
+    uint32_t grown_from = 32;  // the table that filled last
     for (;;) {
         ++attempts;
         int rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
@@ -746,10 +753,18 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
             cudaGetLastError();
             rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
         }
+        if (rc == GASTAR_OUT_OF_MEMORY && table_log2 > grown_from + 1) {  // a smaller step
+            cudaGetLastError();
+            --table_log2;
+            continue;
+        }
         if (rc != GASTAR_OK) return rc;
         if (!cfg.regrow) break;
         if (ctl.status == ST_TABLE_FULL && pp.kind != KIND_GRID && table_log2 < max_log2) {
-            ++table_log2;
+            // Every attempt searches anew, so a table that filled is followed
+            // by one eight times as large.
+            grown_from = table_log2;
+            table_log2 = std::min(max_log2, table_log2 + kRegrowLog2);
             continue;
         }
         if (ctl.status == ST_HEAP_FULL && heap_entries < (1ull << 32)) {
