@@ -111,24 +111,6 @@ const void* search_kernel_for(uint32_t kinds, uint32_t threads) {
     }
 }
 
-uint32_t entry_bytes(uint32_t kind) { return kind == KIND_SLIDING5 ? 32u : 16u; }
-uint32_t max_neighbours(uint32_t kind) { return kind == KIND_GRID ? 8u : 4u; }
-uint32_t key_words(uint32_t kind) { return kind == KIND_SLIDING5 ? 2u : 1u; }
-
-size_t block_smem_bytes(uint32_t kinds, uint32_t warps, uint32_t ew, bool multi, uint32_t heap_snodes,
-                        bool buckets) {
-    // Two stage buffers (one-block teams) + per warp: shared-memory heap
-    // nodes and the bucket push scratch.
-    size_t best = 0;
-    for (uint32_t k = 0; k < 4; ++k)
-        if (kinds & kind_bit(k)) {
-            const size_t stage = multi ? 0 : 2 * stage_entries_per_buffer(warps, ew, max_neighbours(k)) * entry_bytes(k);
-            const size_t per_warp = (size_t)(heap_snodes - 1) * 32 * entry_bytes(k) + (buckets ? 256 : 0);
-            best = std::max(best, stage + ((size_t)warps * per_warp + 15) / 16 * 16);
-        }
-    return best;
-}
-
 uint32_t fit_heap_snodes(gastar_ctx* c, uint32_t kinds, uint32_t warps, uint32_t ew, bool multi, uint32_t threads,
                          int blocks_per_sm, size_t* smem, bool buckets) {
     *smem = block_smem_bytes(kinds, warps, ew, multi, kHeapSmemNodes, buckets);
@@ -434,65 +416,6 @@ struct AttemptStats {
     uint64_t h2d = 0, d2h = 0;
 };
 
-struct PlainShape {
-    uint32_t ew = 0, W = 0;  // pops per warp-heap, warps per block
-    uint64_t blocks = 0;     // 0: no such shape
-    bool cluster = false;
-};
-
-// Shape of a ring team with the automatic widths: eight warps on every SM,
-// popping few entries each.  An iteration lasts as long as its slowest warp,
-// and a warp expands its pops in rounds (four grid cells, eight boards), so
-// many warps with one or two rounds beat fewer with more.  Measured on 152
-// blocks with 16-, 8- and 4-wide pops: 16 15-puzzles 10.6, 8.5 and 9.8 ms
-// (4-wide: too few pops); 1021^2 grid 8.8, 6.9 and 6.2 ms; 4096^2 grid 37.3,
-// 30.6 and 32.8 -- its frontier (~4000 cells) fills 4-wide pops, hence the
-// line at 2^22 cells.
-// Q above 16384 asks for throughput on hard puzzles: pops as wide as it says.
-static PlainShape ring_shape(const gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
-    PlainShape s;
-    const uint64_t warps = 8ull * (uint64_t)c->sms;
-    s.W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block) : 8u;
-    if (cfg.expansion_width) s.ew = std::min(32u, cfg.expansion_width);
-    else if (pp.kind == KIND_GRID) s.ew = (uint64_t)pp.W * pp.H >= (1ull << 22) ? 8 : 4;
-    else s.ew = (uint32_t)std::min<uint64_t>(Q <= 16384 ? 8 : 32, std::max<uint64_t>(4, (Q + warps - 1) / warps));
-    const bool fixed = cfg.expansion_width || cfg.warps_per_block;
-    const uint64_t heaps = std::min<uint64_t>((Q + s.ew - 1) / s.ew, fixed ? ~0ull : warps);
-    s.blocks = (heaps + s.W - 1) / s.W;
-    return s;
-}
-
-// Shape of a team that is one thread-block cluster (or one block), or none.
-// Up to 16 blocks pass their entries and minima through distributed shared
-// memory behind one cluster barrier (~400 cycles) instead of the ring's
-// fences and flags (~2400), but have a tenth of the SMs: taken for searches
-// whose iterations hold a few hundred entries -- Q that small, 8-puzzles
-// (181,440 states in all; 0.167 against 0.196 ms) and grids up to 2^17 cells
-// (200 x 150: 0.92 against 1.12 ms; 360 x 360: 2.18 against 2.13; 517 x 389:
-// 3.03 against 2.81).
-static PlainShape cluster_shape(const PlainProblem& pp, const gastar_config& cfg, uint64_t Q) {
-    PlainShape s;
-    const bool fixed = cfg.expansion_width || cfg.warps_per_block;
-    s.W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block) : 8u;
-    s.ew = cfg.expansion_width ? std::min(32u, cfg.expansion_width) : 4u;
-    if (s.W > 8) return PlainShape();  // their kernel has no cluster teams for single instances
-    const bool few = pp.kind == KIND_SLIDING3 || (pp.kind == KIND_GRID && (uint64_t)pp.W * pp.H <= (1ull << 17));
-    uint64_t blocks = (Q + (uint64_t)s.ew * s.W - 1) / ((uint64_t)s.ew * s.W);
-    if (blocks > kMaxClusterBlocks) {
-        if (fixed || !few) return PlainShape();
-        blocks = kMaxClusterBlocks;
-    }
-    if (cfg.max_blocks) blocks = std::min<uint64_t>(blocks, cfg.max_blocks);
-    s.cluster = blocks > 1;
-    if (s.cluster) {
-        const uint32_t kinds = kind_bit(pp.kind);
-        const size_t smem = block_smem_bytes(kinds, s.W, s.ew, false, kHeapSmemNodes, cfg.open_list == 1);
-        if (occupancy_clusters(kinds, s.W * 32, smem, (uint32_t)blocks) < 1) return PlainShape();
-    }
-    s.blocks = blocks;
-    return s;
-}
-
 // A search whose table fills starts again in one of 2^kRegrowLog2 times the
 // slots.  64 15-puzzles (walk 20-80, Q = 4096), three of which fill the first
 // table, take 105 ms with doubling (up to four searches), 80.5 with 2, 60.8
@@ -505,41 +428,34 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
                          cudaStream_t st, InstCtl& ctl_out, AttemptStats& as) {
     const bool want_path = path_keys != nullptr;
     const uint32_t kinds = kind_bit(pp.kind);
-    const uint64_t Q = cfg.num_queues ? cfg.num_queues : 4096;
-    PlainShape sh = cluster_shape(pp, cfg, Q);
-    if (!sh.blocks) sh = ring_shape(c, pp, cfg, Q);
+    const bool buckets = cfg.open_list == 1;
+    PlainShape sh = plain_shape((uint32_t)c->sms, pp.kind, (uint64_t)pp.W * pp.H, cfg,
+                                [&](uint32_t warps, uint32_t ew, uint32_t blocks) {
+                                    const size_t smem =
+                                        block_smem_bytes(kinds, warps, ew, false, kHeapSmemNodes, buckets);
+                                    return occupancy_clusters(kinds, warps * 32, smem, blocks) >= 1;
+                                });
     const uint32_t ew = sh.ew, W = sh.W, threads = W * 32;
-    uint64_t blocks = sh.blocks, heaps = blocks * W;
-    const bool cluster = sh.cluster, multi = blocks > 1 && !cluster;  // multi: a ring team
-    // Widening: a puzzle search with the automatic width that passes
-    // kWideAfter iterations is a hard one, whose iteration count the pops per
-    // iteration set rather than its depth; from then on every warp-heap pops
-    // four times as many (at most 32).  On the 64 15-puzzles of the plain
-    // benchmark (Q = 16384, 8-wide pops) the hardest took 333 iterations with
-    // twice the pops and takes 206 with four times; the 64 together 4 % less
-    // time.
-    const uint32_t ew_wide =
-        multi && pp.kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 4 * ew) : ew;
-    size_t smem = block_smem_bytes(kinds, W, ew, multi);
+    size_t smem = block_smem_bytes(kinds, W, ew, sh.ring());
     const int nb = occupancy_blocks(c, kinds, threads, smem);
     if (nb <= 0) return GASTAR_CUDA_ERROR;
-    uint64_t max_blocks = (uint64_t)nb * c->sms;
-    if (cfg.max_blocks) max_blocks = std::min<uint64_t>(max_blocks, cfg.max_blocks);
-    if (blocks > max_blocks) blocks = max_blocks;
+    sh.blocks = std::min(sh.blocks, (uint64_t)nb * c->sms);
+    sh.ew_wide = widened(sh, pp.kind, cfg);
+    const uint64_t blocks = sh.blocks, heaps = blocks * W;
+    const bool cluster = sh.cluster, ring = sh.ring();
+    const uint32_t ew_wide = sh.ew_wide;
     // The shared memory the co-resident blocks leave free holds the heaps' top
     // levels: pops and pushes then touch global nodes only deep down.
-    const bool buckets = cfg.open_list == 1;
-    uint32_t snodes = fit_heap_snodes(c, kinds, W, ew, multi, threads,
+    uint32_t snodes = fit_heap_snodes(c, kinds, W, ew, ring, threads,
                                             (int)((blocks + c->sms - 1) / c->sms), &smem, buckets);
     if (cluster && occupancy_clusters(kinds, threads, smem, (uint32_t)blocks) < 1) {
-        smem = block_smem_bytes(kinds, W, ew, multi, kHeapSmemNodes, buckets);
+        smem = block_smem_bytes(kinds, W, ew, ring, kHeapSmemNodes, buckets);
         snodes = kHeapSmemNodes;
     }
-    if (multi && !c->coop) {
+    if (ring && !c->coop) {
         set_error("device does not support cooperative launch");
         return GASTAR_CUDA_ERROR;
     }
-    heaps = blocks * W;
     const uint32_t maxn = max_neighbours(pp.kind);
 
     // Duplicate-detection table: a dense per-cell array for grids (cleared by
@@ -585,7 +501,7 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     uint64_t cap_nodes = std::max<uint64_t>(2 * snodes, (per_heap * 2 + 31) / 32);
     if (cap_nodes > 0x7fffffffull) return GASTAR_OUT_OF_MEMORY;
     const size_t heap_bytes = (size_t)heaps * (cap_nodes + 1) * 32 * ebytes;
-    const size_t stage_bytes = multi ? team_stage_bytes((uint32_t)blocks, W, ew_wide, maxn, ebytes) : 16;
+    const size_t stage_bytes = ring ? team_stage_bytes((uint32_t)blocks, W, ew_wide, maxn, ebytes) : 16;
 
     if (!c->heaps.ensure(heap_bytes) || !c->hdr.ensure((size_t)heaps * 8) ||
         !c->stage.ensure(stage_bytes) || !c->launch.ensure(kLbBytes))

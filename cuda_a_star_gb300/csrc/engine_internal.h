@@ -10,6 +10,7 @@
 
 #include "../../include/gastar.h"
 #include "engine_types.h"
+#include "team_shape.h"
 
 namespace gastar {
 
@@ -54,11 +55,6 @@ const void* search_kernel_grid();
 const void* search_kernel_all();
 const void* search_kernel_all16();
 const void* search_kernel_for(uint32_t kinds, uint32_t threads);
-uint32_t entry_bytes(uint32_t kind);
-uint32_t max_neighbours(uint32_t kind);
-uint32_t key_words(uint32_t kind);
-size_t block_smem_bytes(uint32_t kinds, uint32_t warps, uint32_t ew, bool multi,
-                        uint32_t heap_snodes = kHeapSmemNodes, bool buckets = false);
 int launch_search(struct ::gastar_ctx* c, uint32_t kinds, const LaunchParams& P, uint32_t blocks,
                   uint32_t threads, size_t smem, cudaStream_t st);
 // Rebuilds the paths of finished instances into `arena` (see path_kernel):
