@@ -26,6 +26,9 @@ enum : uint32_t {
     ST_OK = 0, ST_NO_PATH = 1, ST_BUDGET = 2, ST_TIMEOUT = 3, ST_HEAP_FULL = 4,
     ST_TABLE_FULL = 5, ST_PATH_CAP = 6, ST_BARRIER = 7, ST_BAD_INPUT = 8, ST_COST_RANGE = 13,
 };
+static_assert(ST_HEAP_FULL > ST_BUDGET && ST_HEAP_FULL > ST_TIMEOUT && ST_TABLE_FULL > ST_HEAP_FULL &&
+                  ST_COST_RANGE > ST_TABLE_FULL,
+              "an iteration's status is the largest code raised: lost entries before budgets");
 enum : uint32_t { LIFE_FRESH = 0, LIFE_RUNNING = 1, LIFE_DONE = 2 };
 
 __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {

@@ -146,7 +146,10 @@ struct alignas(16) TeamSlot {
     uint32_t count;     // entries staged in the pop/expand phase
     uint32_t minstage;  // least f of the entries staged
     uint32_t best;      // goal costs found in the pop/expand phase
-    uint32_t err;       // first error raised in the pop/expand phase
+    // Largest status raised in the pop/expand phase.  Lost entries (heap full,
+    // table full, cost range) have larger codes than budgets and timeouts, so
+    // that a budget in the same iteration never hides them.
+    uint32_t err;
     // The other blocks of a cluster read the two halves as 16 bytes each.
     uint32_t claims;    // table slots claimed
     uint32_t exps;      // entries expanded

@@ -721,11 +721,12 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             }
         }
         if (!ring && leader) {
-            if (sm.base[0] + sm.run[0] > d.table_limit) atomicCAS(&S->err, 0u, (uint32_t)ST_TABLE_FULL);
-            if (d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
-            if (d.max_iter && it0 + it + 1 >= d.max_iter) atomicCAS(&S->err, 0u, (uint32_t)ST_BUDGET);
-            if (d.timeout_ns && globaltimer_ns() - sm.t_start > d.timeout_ns)
-                atomicCAS(&S->err, 0u, (uint32_t)ST_TIMEOUT);
+            uint32_t err = 0;
+            if (sm.base[0] + sm.run[0] > d.table_limit) err = ST_TABLE_FULL;
+            else if (d.max_exp && sm.base[1] + sm.run[1] >= d.max_exp) err = ST_BUDGET;
+            else if (d.max_iter && it0 + it + 1 >= d.max_iter) err = ST_BUDGET;
+            else if (d.timeout_ns && globaltimer_ns() - sm.t_start > d.timeout_ns) err = ST_TIMEOUT;
+            if (err) atomicMax(&S->err, err);
         }
 
         // ---- pop: up to ew entries per warp-heap, inside the window ----
@@ -952,8 +953,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 if (n_claim) atomicAdd(&Sw->claims, n_claim);
                 if (smin != kInf) atomicMin(&Sw->minstage, smin);
                 if (goal_g != kInf) atomicMin(&Sw->best, goal_g);
-                if (flags & 1u) atomicCAS(&Sw->err, 0u, (uint32_t)ST_TABLE_FULL);
-                if (flags & 2u) atomicCAS(&Sw->err, 0u, (uint32_t)ST_COST_RANGE);
+                if (flags & 1u) atomicMax(&Sw->err, (uint32_t)ST_TABLE_FULL);
+                if (flags & 2u) atomicMax(&Sw->err, (uint32_t)ST_COST_RANGE);
             }
         }
         if constexpr (ring) {
@@ -1095,7 +1096,6 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                     }
                     if (!have_prev) q.z = kInf, q.w = 0;
                     const uint32_t b_min = __reduce_min_sync(kFull, a.z);
-                    // The largest code wins: lost entries before budgets.
                     const uint32_t e_max = __reduce_max_sync(kFull, a.w > q.w ? a.w : q.w);
                     const uint32_t f_min = __reduce_min_sync(kFull, a.y < q.z ? a.y : q.z);
                     if (rank == 0) {  // the team's counts, for the budgets
@@ -1141,7 +1141,7 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 open_f = uniform(ld_vol(&S->minstage));
                 if (have_prev) {
                     const uint32_t pe = uniform(ld_vol(&pv->perr)), mf = uniform(ld_vol(&pv->minheap));
-                    if (!err) err = pe;
+                    err = pe > err ? pe : err;
                     open_f = mf < open_f ? mf : open_f;
                 }
             }
