@@ -383,11 +383,12 @@ int batch_upload(gastar_batch* b) {
         }
     }
     // Teams are clusters (a grid of whole clusters) where as many blocks are
-    // resident that way.
+    // resident that way and the caller's cap admits them.
     b->cluster = false;
     if (b->n_heavy && cluster_team_size(T)) {
         const uint32_t whole = (b->blocks + T - 1) / T;
-        if ((uint32_t)occupancy_clusters(kKindsAll, b->threads, b->smem, T) >= whole) {
+        if ((!b->cfg.blocks || whole * T <= b->cfg.blocks) &&
+            (uint32_t)occupancy_clusters(kKindsAll, b->threads, b->smem, T) >= whole) {
             b->cluster = true;
             b->blocks = whole * T;
         }
