@@ -403,7 +403,9 @@ int batch_upload(gastar_batch* b) {
         arena_bytes += plans[i].bytes;
         b->path_words += plans[i].path_words;
     }
-    if (!c->spare.take(b->arena, arena_bytes, SPARE_ARENA)) {
+    // An upload that failed further on left its arena: taken again as it is.
+    if (b->arena.n < arena_bytes) b->arena.release();
+    if (!b->arena.p && !c->spare.take(b->arena, arena_bytes, SPARE_ARENA)) {
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
         if (arena_bytes + (64ull << 20) > free_b) {
