@@ -172,13 +172,9 @@ uint8_t* grid_alloc(gastar_batch* b, size_t bytes) {
     if (b->grid_chunks.empty() || b->grid_chunk_used + bytes > b->grid_chunk_cap) {
         const size_t cap = std::max<size_t>(bytes, (size_t)256 << 20);
         DevBuf c;
-        if (!b->ctx->spare.take(c, cap, SPARE_GRIDS) && !c.ensure(cap)) {
-            b->ctx->spare.drop();
+        if (!b->ctx->batch_memory.take(c, cap, b->ctx->stream)) {
             cudaGetLastError();
-            if (!c.ensure(cap)) {
-                cudaGetLastError();
-                return nullptr;
-            }
+            return nullptr;
         }
         b->grid_chunks.push_back(c);
         b->grid_chunk_cap = c.n;
@@ -235,8 +231,8 @@ void gastar_batch_destroy(gastar_batch* b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     gastar_batch_destroy(b->sub);
     // The stream is idle: the next batch of this context may have the memory.
-    b->ctx->spare.give(b->arena, SPARE_ARENA);
-    for (DevBuf& c : b->grid_chunks) b->ctx->spare.give(c, SPARE_GRIDS);
+    b->ctx->batch_memory.give(b->arena, b->ctx->stream);
+    for (DevBuf& c : b->grid_chunks) b->ctx->batch_memory.give(c, b->ctx->stream);
     b->descs.release();
     b->ctls.release();
     b->order.release();
@@ -404,24 +400,19 @@ int batch_upload(gastar_batch* b) {
         b->path_words += plans[i].path_words;
     }
     // An upload that failed further on left its arena: taken again as it is.
-    if (b->arena.n < arena_bytes) b->arena.release();
-    if (!b->arena.p && !c->spare.take(b->arena, arena_bytes, SPARE_ARENA)) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        if (arena_bytes + (64ull << 20) > free_b) {
-            c->spare.drop();
-            cudaMemGetInfo(&free_b, &total_b);
-        }
-        if (arena_bytes + (64ull << 20) > free_b) {
+    if (b->arena.n < arena_bytes) c->batch_memory.give(b->arena, c->stream);
+    if (!b->arena.p) {
+        if (!c->batch_memory.room(arena_bytes + (64ull << 20))) {
             set_error("batch partitions exceed free device memory");
             return GASTAR_OUT_OF_MEMORY;
         }
+        if (!c->batch_memory.take(b->arena, arena_bytes, c->stream)) return GASTAR_OUT_OF_MEMORY;
     }
-    if (!b->arena.ensure(arena_bytes) || !b->descs.ensure(sizeof(InstDesc) * n) || !b->ctls.ensure(sizeof(InstCtl) * (n + 1)) ||
+    if (!b->descs.ensure(sizeof(InstDesc) * n) || !b->ctls.ensure(sizeof(InstCtl) * (n + 1)) ||
         !b->order.ensure(sizeof(uint32_t) * n) || !b->counters.ensure(64) ||
         !b->paths.ensure(b->path_words * 8) || !b->tcounts.ensure(sizeof(unsigned long long) * n))
         return GASTAR_OUT_OF_MEMORY;
-    b->device_bytes = arena_bytes + b->grid_bytes + b->path_words * 8 +
+    b->device_bytes = b->arena.n + b->grid_bytes + b->path_words * 8 +
                       (sizeof(InstDesc) + sizeof(InstCtl)) * (size_t)n;
     char* base = reinterpret_cast<char*>(b->arena.p);
     InstCtl* ctl_base = reinterpret_cast<InstCtl*>(b->ctls.p);

@@ -57,6 +57,7 @@ void DevBuf::release() {
     if (p) cudaFree(p);
     p = nullptr;
     n = 0;
+    pooled = false;
 }
 
 bool DevBuf::ensure(size_t bytes) {
@@ -73,31 +74,80 @@ bool DevBuf::ensure(size_t bytes) {
     return true;
 }
 
-bool SpareMemory::take(DevBuf& b, size_t bytes, int which) {
+bool BatchMemory::take(DevBuf& b, size_t bytes, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(mu_);
-    DevBuf& k = kept_[which];
-    if (!k.p || k.n < bytes) return false;
-    b = k;
-    b.fresh = true;
-    k = DevBuf();
+    if (!again_ || bytes > kKeepMax) return b.ensure(bytes);
+    if (!pool_) {
+        int dev = 0;
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        uint64_t keep = kKeepMax;
+        if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return false;
+        props.location.id = dev;
+        if (!cuda_ok(cudaMemPoolCreate(&pool_, &props), "cudaMemPoolCreate")) {
+            pool_ = nullptr;
+            return false;
+        }
+        if (!cuda_ok(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep),
+                     "cudaMemPoolSetAttribute"))
+            return false;
+    }
+    void* p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, pool_, st) != cudaSuccess) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool_, 0);  // kept, but in pieces
+        if (!cuda_ok(cudaMallocFromPoolAsync(&p, bytes, pool_, st), "cudaMallocFromPoolAsync")) return false;
+    }
+    // Complete when it returns, so that the buffer may be used on any stream.
+    if (!cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize")) return false;
+    b.p = p;
+    b.n = bytes;
+    b.fresh = b.pooled = true;
     return true;
 }
 
-void SpareMemory::give(DevBuf& b, int which) {
+void BatchMemory::give(DevBuf& b, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(mu_);
-    DevBuf& k = kept_[which];
-    if (b.p && b.n <= kSpareMax && b.n > k.n) std::swap(b, k);
-    b.release();
+    if (!b.p) return;
+    again_ = true;
+    if (!b.pooled) {
+        b.release();
+        return;
+    }
+    cuda_ok(cudaFreeAsync(b.p, st), "cudaFreeAsync");
+    cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    b = DevBuf();
 }
 
-bool SpareMemory::drop() {
+void BatchMemory::trim() {
     std::lock_guard<std::mutex> lk(mu_);
-    bool any = false;
-    for (DevBuf& k : kept_) {
-        any = any || k.p;
-        k.release();
+    if (pool_) cuda_ok(cudaMemPoolTrimTo(pool_, 0), "cudaMemPoolTrimTo");
+}
+
+void BatchMemory::close() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (pool_) cuda_ok(cudaMemPoolDestroy(pool_), "cudaMemPoolDestroy");
+    pool_ = nullptr;
+}
+
+bool BatchMemory::room(size_t bytes) {
+    std::lock_guard<std::mutex> lk(mu_);
+    size_t free_b = 0, total_b = 0;
+    uint64_t held = 0, used = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    if (pool_) {
+        cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &held);
+        cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrUsedMemCurrent, &used);
     }
-    return any;
+    if (bytes <= free_b + (held - used)) return true;
+    void* p = nullptr;  // other contexts' pools: what cudaMalloc gets of them
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaFree(p);
+    return true;
 }
 
 const void* search_kernel_for(uint32_t kinds, uint32_t threads) {
@@ -372,7 +422,7 @@ void gastar_destroy(gastar_ctx* c) {
     c->path.release();
     c->misc.release();
     c->weights.release();
-    c->spare.drop();
+    c->batch_memory.close();
     destroy_stager(c->stager);
     if (c->h_ctl) cudaFreeHost(c->h_ctl);
     if (c->h_launch) cudaFreeHost(c->h_launch);
@@ -665,10 +715,6 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
     for (;;) {
         ++attempts;
         int rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
-        if (rc == GASTAR_OUT_OF_MEMORY && c->spare.drop()) {  // again without what was kept for batches
-            cudaGetLastError();
-            rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
-        }
         if (rc == GASTAR_OUT_OF_MEMORY && table_log2 > grown_from + 1) {  // a smaller step
             cudaGetLastError();
             --table_log2;

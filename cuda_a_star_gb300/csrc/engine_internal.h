@@ -18,31 +18,39 @@ struct DevBuf {
     void* p = nullptr;
     size_t n = 0;
     bool fresh = false;         // set when ensure() reallocated (contents undefined)
+    bool pooled = false;        // from a memory pool (BatchMemory)
     bool ensure(size_t bytes);  // grows (contents are not kept)
     void release();
 };
 
-// Device memory of a destroyed batch, kept by its context for the next one:
-// mapping and unmapping a batch's partitions (11 GB for 512 8-puzzles) takes
-// longer than searching them.  One partition arena and one chunk of grid
-// weights, at most kSpareMax bytes each; whatever else of this library finds
-// too little memory on the device takes them back first (drop), and the
-// context's end releases them.
-class SpareMemory {
+// Device memory for batches that a context's later batches use again: mapping
+// and unmapping a batch's partitions (11 GB for 512 8-puzzles: 1.3 and 4.9 ms)
+// takes longer than searching them (1.9 ms).  What a destroyed batch gives back
+// stays in a memory pool of the driver, at most kKeepMax bytes, which hands it
+// out in exact sizes and takes it back by itself for any cudaMalloc of the
+// process that would fail, whoever calls it (20 ms for 8 GB).  Growing a pool
+// takes longer than cudaMalloc (0.8 against 0.1 ms per GB, and 0.4 to free), so
+// the first batch of a context, and buffers above kKeepMax, go without it.
+class BatchMemory {
 public:
-    static constexpr size_t kSpareMax = (size_t)16 << 30;
-    // Moves a kept buffer of at least `bytes` into `b` (empty); false: none.
-    bool take(DevBuf& b, size_t bytes, int which);
-    // Keeps `b`, or what was kept if that is larger, and releases the other.
-    void give(DevBuf& b, int which);
-    // Releases what is kept; false: nothing was.
-    bool drop();
+    static constexpr size_t kKeepMax = (size_t)16 << 30;
+    // Allocates `bytes` into `b` (empty) for work on `st`, which is idle.
+    bool take(DevBuf& b, size_t bytes, cudaStream_t st);
+    // Releases `b`; the work that used it is done.
+    void give(DevBuf& b, cudaStream_t st);
+    // Whether a batch may take `bytes`: what is kept unused, here or by other
+    // contexts of the process, counts as free; the latter's is free after it
+    // where it was needed.
+    bool room(size_t bytes);
+    // Gives what is kept unused back to the device.
+    void trim();
+    void close();
 
 private:
     std::mutex mu_;
-    DevBuf kept_[2];
+    cudaMemPool_t pool_ = nullptr;
+    bool again_ = false;  // a batch has been destroyed
 };
-enum { SPARE_ARENA = 0, SPARE_GRIDS = 1 };
 
 void set_error(const std::string& s);
 bool cuda_ok(cudaError_t e, const char* what);
@@ -134,7 +142,7 @@ struct gastar_ctx {
     bool can_read_host = false;    // kernels read pageable host memory through the host's
                                    // page tables (ATS over NVLink-C2C on Grace)
     int upload_mode = 2;           // grid uploads: 0 copy, 1 read in place, 2 staged
-    gastar::SpareMemory spare;
+    gastar::BatchMemory batch_memory;
     gastar::HostStager* stager = nullptr;  // staged uploads (pinned ring, host threads)
     bool table_dirty = true;       // hash table needs a full clear before the next solve
     uint32_t prev_slot_words = 2;  // slot width of the solve that filled the touched list

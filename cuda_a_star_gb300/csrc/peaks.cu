@@ -87,7 +87,6 @@ int measure(gastar_ctx* ctx, uint64_t bytes, uint32_t kind, uint32_t in_flight, 
     if (cudaSetDevice(ctx->device) != cudaSuccess) return GASTAR_CUDA_ERROR;
     void* buf = nullptr;
     unsigned long long* sink = nullptr;
-    ctx->spare.drop();
     if (cudaMalloc(&buf, bytes) != cudaSuccess) return GASTAR_OUT_OF_MEMORY;
     if (cudaMalloc(&sink, 8) != cudaSuccess) {
         cudaFree(buf);

@@ -329,10 +329,13 @@ gastar_server* gastar_serve_create(gastar_ctx* c, const gastar_serve_config* cfg
     cf.expansion_width = std::min(32u, cf.expansion_width);
     if (cf.load_factor <= 0.f) cf.load_factor = 0.75f;
     if (!cf.slice_iters) cf.slice_iters = 128;
-    c->spare.drop();  // the budget is a share of the memory that is free
+    uint64_t budget = cf.budget_bytes ? cf.budget_bytes : (120ull << 30);
+    // The budget is a share of the memory that is free, what contexts keep
+    // for batches included.
+    c->batch_memory.trim();
+    c->batch_memory.room(budget + (2ull << 30));
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    uint64_t budget = cf.budget_bytes ? cf.budget_bytes : (120ull << 30);
     budget = std::min<uint64_t>(budget, free_b > (2ull << 30) ? free_b - (2ull << 30) : free_b / 2);
     cf.budget_bytes = budget;
     s->threads = cf.warps_per_block * 32;

@@ -198,6 +198,10 @@ typedef struct gastar_batch_config {
 
 void gastar_batch_config_default(gastar_batch_config *cfg);
 gastar_batch *gastar_batch_create(gastar_ctx *ctx, const gastar_batch_config *cfg);
+/* The partitions' and grids' memory stays with the context for its later
+ * batches, at most 16 GiB of it, in a memory pool whose unused part the driver
+ * gives to any allocation of the process that would fail otherwise.
+ * gastar_serve_create and gastar_destroy return it to the device. */
 void gastar_batch_destroy(gastar_batch *b);
 /* Returns the instance index (>= 0) or a negative gastar_status. */
 int gastar_batch_add_sliding(gastar_batch *b, uint32_t n, const uint8_t *start,

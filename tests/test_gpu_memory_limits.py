@@ -65,3 +65,105 @@ def test_a_batch_that_ran_out_of_memory_runs_later_and_leaks_nothing(gastar):
             b.close()
         after = _free()
     assert after >= before - 64 * MIB
+
+
+def _puzzles(eng, gastar, count):
+    """15-puzzles, whose partitions take about 100 MB each."""
+    b = eng.batch()
+    for i in range(count):
+        b.add_sliding(*gastar.gen_sliding(4, 700 + i, 20, 24))
+    return b
+
+
+@pytest.fixture()
+def kept(gastar):
+    """An engine, and the bytes it holds after batches were closed."""
+    with gastar.Engine(0) as eng:
+        s, g = gastar.gen_sliding(4, 1, 20, 24)
+        eng.solve_sliding(s, g, 4)
+        before = _free()
+        for _ in range(3):
+            b = _puzzles(eng, gastar, 40)
+            b.run()
+            b.close()
+        yield eng, before - _free()
+
+
+def test_memory_kept_after_a_batch_serves_torch(kept):
+    import torch
+    eng, held = kept
+    assert held > 2 << 30  # what this is about
+    hog = _fill(512 * MIB)
+    more = torch.empty(held - 512 * MIB, dtype=torch.uint8, device="cuda")  # more than is free
+    del hog, more
+    _free()
+
+
+def test_memory_kept_after_a_batch_serves_the_library(kept, gastar):
+    """Uploads, another context's solves and batches, and batches of the same
+    context, when the rest of the device is taken."""
+    import numpy as np
+    eng, held = kept
+    assert held > 2 << 30
+    grid = np.full((20000, 50000), 3, dtype=np.uint8)  # 1 GB
+    hog = _fill(512 * MIB)
+    assert eng.grid_min_weight(grid)[0] == 3
+    del hog
+    _free()
+    for _ in range(2):
+        b = _puzzles(eng, gastar, 40)
+        b.run()
+        b.close()
+    with gastar.Engine(0) as other:
+        hog = _fill(512 * MIB)
+        s, g = gastar.gen_sliding(4, 2, 20, 24)
+        want = eng.solve_sliding(s, g, 4).cost
+        r = other.solve_sliding(s, g, 4, table_log2=26)  # a 1 GiB table
+        assert r.status_name == "OK" and r.cost == want
+        b = _puzzles(other, gastar, 10)
+        b.run()
+        assert all(b.result(i).status_name == "OK" for i in range(len(b)))
+        b.close()
+        del hog
+        _free()
+
+
+def test_a_small_batch_leaves_the_rest_of_what_is_kept(kept, gastar):
+    import torch
+    eng, held = kept
+    b = _puzzles(eng, gastar, 2)
+    b.run()
+    took = b.stats()["device_bytes"]
+    assert took < 512 * MIB
+    hog = _fill(512 * MIB)
+    more = torch.empty(held - took - 512 * MIB, dtype=torch.uint8, device="cuda")
+    assert b.result(0).status_name == "OK"
+    b.rerun()
+    assert b.result(0).status_name == "OK"
+    del hog, more
+    _free()
+    b.close()
+
+
+def test_batches_use_what_is_kept_when_the_device_is_full(kept, gastar):
+    eng, held = kept
+    hog = _fill(600 * MIB)
+    for count in (40, 7, 40):
+        b = _puzzles(eng, gastar, count)
+        b.run()
+        assert all(b.result(i).status_name == "OK" for i in range(count))
+        b.close()
+    del hog
+    _free()
+
+
+def test_a_servers_budget_counts_what_another_context_keeps(kept, gastar):
+    eng, held = kept
+    with gastar.Engine(0) as other:
+        free = _free()
+        budget = free + held - (3 << 30)
+        srv = other.server(budget_bytes=budget, weights_pool=0)
+        assert _free() <= free + held - budget
+        i = srv.submit_sliding(*gastar.gen_sliding(3, 9, 20, 24))
+        assert srv.drain([i])[i].status_name == "OK"
+        srv.close()
