@@ -471,6 +471,16 @@ struct AttemptStats {
 // table, take 105 ms with doubling (up to four searches), 80.5 with 2, 60.8
 // with 3, 58.7 with 4, which may take twice the memory for that.
 constexpr uint32_t kRegrowLog2 = 3;
+// Such a table is kept for later solves unless it is this much larger than the
+// one doubling would have ended with, and than any that was there before.
+constexpr size_t kRegrowKeep = (size_t)1 << 30;
+
+static uint32_t slot_words(uint32_t kind) { return key_words(kind) == 1 ? 2 : 4; }
+// Claimed slots a table of 2^log2 may hold.
+static uint64_t table_limit(uint32_t log2, const gastar_config& cfg) {
+    const float lf = cfg.load_factor > 0.f ? cfg.load_factor : 0.75f;
+    return (uint64_t)((double)(1ull << log2) * std::min(0.95f, std::max(0.1f, lf)));
+}
 
 // Runs the search (+ path rebuild) once with the given capacities.
 static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_config& cfg,
@@ -512,7 +522,7 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     // the kernel), a hash table for puzzles that stays allocated across solves
     // and is cleared slot by slot from the previous solve's claim list.
     const uint32_t ebytes = entry_bytes(pp.kind), kw = key_words(pp.kind);
-    const uint32_t slot_words = kw == 1 ? 2 : 4;
+    const uint32_t sw = slot_words(pp.kind);
     uint64_t table_words, mask = 0, limit = ~0ull, touched_cap = 0;
     DevBuf* tb;
     if (pp.kind == KIND_GRID) {
@@ -521,11 +531,9 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
         if (!tb->ensure(table_words * 8)) return GASTAR_OUT_OF_MEMORY;
     } else {
         const uint64_t slots = 1ull << table_log2;
-        table_words = slots * slot_words;
+        table_words = slots * sw;
         mask = slots - 1;
-        float lf = cfg.load_factor > 0.f ? cfg.load_factor : 0.75f;
-        lf = std::min(0.95f, std::max(0.1f, lf));
-        limit = (uint64_t)((double)slots * lf);
+        limit = table_limit(table_log2, cfg);
         // Claims stop within two iterations past the limit; every warp may
         // leave one chunk partly unused.
         touched_cap = limit + 2 * heaps * ew_wide * maxn + heaps * kTouchedChunk + 16;
@@ -650,7 +658,7 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     GA_CUDA(cudaStreamSynchronize(st));
     as.d2h += sizeof(InstCtl);
     if (pp.kind != KIND_GRID) {
-        c->prev_slot_words = slot_words;
+        c->prev_slot_words = sw;
         // Reserved entries <= 1 + claims + one chunk per warp: beyond the
         // list's size some claims went unrecorded.
         if (1 + c->h_ctl->table_used + heaps * kTouchedChunk > touched_cap) c->table_dirty = true;
@@ -712,12 +720,14 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
     AttemptStats as;
     uint32_t attempts = 0;
     uint32_t grown_from = 32;  // the table that filled last
+    const size_t held = c->table.n;
     for (;;) {
         ++attempts;
         int rc = plain_attempt(c, pp, cfg, table_log2, heap_entries, path_keys, st, ctl, as);
         if (rc == GASTAR_OUT_OF_MEMORY && table_log2 > grown_from + 1) {  // a smaller step
             cudaGetLastError();
             --table_log2;
+            --attempts;  // nothing was searched
             continue;
         }
         if (rc != GASTAR_OK) return rc;
@@ -734,6 +744,15 @@ int plain_solve(gastar_ctx* c, const PlainProblem& pp, const gastar_config* user
             continue;
         }
         break;
+    }
+    if (grown_from < 32 && ctl.status != ST_TABLE_FULL) {
+        uint32_t log2 = grown_from + 1;  // where doubling would have ended
+        while (log2 < table_log2 && ctl.table_used > table_limit(log2, cfg)) ++log2;
+        const size_t doubled = (size_t)8 * slot_words(pp.kind) << log2;
+        if (c->table.n > std::max(held, doubled + kRegrowKeep)) {
+            c->table.release();
+            c->touched.release();
+        }
     }
     fill_result(out, ctl);
     out->kernel_ms = as.kernel_ms;

@@ -167,3 +167,32 @@ def test_a_servers_budget_counts_what_another_context_keeps(kept, gastar):
         i = srv.submit_sliding(*gastar.gen_sliding(3, 9, 20, 24))
         assert srv.drain([i])[i].status_name == "OK"
         srv.close()
+
+
+def test_a_regrown_table_far_larger_than_needed_is_not_kept(gastar, oracle):
+    """2^24 slots with a limit of a tenth of them, then eight times as many
+    (2 GiB) where twice would have done."""
+    kw = dict(table_log2=24, load_factor=0.1)
+    with gastar.Engine(0) as eng:
+        for walk in range(16, 30):  # boards whose blind search claims 1.8 to 3.2 M states
+            s, g = gastar.gen_sliding(4, 800 + walk, walk, walk)
+            claims = eng.solve_sliding(s, g, 4, heuristic=gastar.H_ZERO, table_log2=26).table_used
+            if 1_800_000 < claims < 3_200_000:
+                break
+        assert 1_800_000 < claims < 3_200_000
+    want = oracle.sliding_astar(4, s, g, path=False)[0].cost
+    easy = gastar.gen_sliding(4, 1, 20, 24)
+    with gastar.Engine(0) as eng:
+        cost = eng.solve_sliding(*easy, 4, **kw).cost
+        before = _free()
+        for _ in range(2):
+            r = eng.solve_sliding(s, g, 4, heuristic=gastar.H_ZERO, **kw)
+            assert r.status_name == "OK" and r.cost == want and r.attempts == 2
+            assert _free() > before - 1024 * MIB  # 2 GiB and its claim list before
+            assert eng.solve_sliding(*easy, 4, **kw).cost == cost
+    with gastar.Engine(0) as eng:  # a table that the caller asked for stays
+        eng.solve_sliding(*easy, 4, table_log2=27)
+        before = _free()
+        r = eng.solve_sliding(s, g, 4, heuristic=gastar.H_ZERO, **kw)
+        assert r.cost == want and r.attempts == 2
+        assert abs(_free() - before) < 256 * MIB
