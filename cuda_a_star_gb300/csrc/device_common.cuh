@@ -71,6 +71,15 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // compiler takes what a load, a shuffle or threadIdx yields for per-lane data
 // and guards every branch on it with convergence code; the result of a
 // reduction or a vote is uniform to it, and so are the branches.
+//
+// Rule: no vote or reduction may have an operand that is a compile-time constant
+// in any instantiation; code that some domains never run goes under `if
+// constexpr`.  A vote on a constant (grids: a flag that only hash tables raise)
+// left all lanes of every warp waiting on the GPU.  Its source was well formed:
+// the lanes of a warp came to every full-mask operation together when the same
+// code was run on the host, and every branch around one is on a vote's or a
+// reduction's result.  So it is kept out by a test that compiles every
+// instantiation for the host (tests/test_vote_predicates.py).
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __reduce_or_sync(kFull, v); }
 __device__ __forceinline__ bool uniform_if(bool c) { return __any_sync(kFull, c) != 0; }
 

@@ -941,8 +941,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
             // reduction each.
             const uint32_t smin = __reduce_min_sync(kFull, fstage);
             goal_g = __reduce_min_sync(kFull, goal_g);
-            // One reduction for both flags.  (Not a vote each: the first is a
-            // constant for grids, and a vote on a constant here hung the warp.)
+            // One reduction for both flags, not a vote each: grids never raise
+            // the first (the rule at uniform()).
             flags = uniform(flags);
             if (lane == 0) {
                 const uint32_t n_exp = __popc(live) - (D::kParentBySlot ? 0u : n_stale);
