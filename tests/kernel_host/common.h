@@ -2,10 +2,18 @@
 // that do not depend on what a warp operation does here.
 #pragma once
 
+// The library's headers come first: they use names that are macros below.
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <memory>
+#include <random>
+#include <type_traits>
+#include <vector>
 
 #define __device__
 #define __host__
