@@ -44,16 +44,19 @@ struct PlainShape {
 // and a warp expands its pops in rounds (four grid cells, eight boards), so
 // many warps with one or two rounds beat fewer with more.  Measured on 152
 // blocks with 16-, 8- and 4-wide pops: 16 15-puzzles 10.6, 8.5 and 9.8 ms
-// (4-wide: too few pops); 1021^2 grid 8.8, 6.9 and 6.2 ms; 4096^2 grid 37.3,
-// 30.6 and 32.8 -- its frontier (~4000 cells) fills 4-wide pops, hence the
-// line at 2^22 cells.
+// (4-wide: too few pops).  Grids pop 4 until their frontier (4096^2: ~4000
+// cells) fills such pops, which with a pop window of 72 it does first; calls
+// with 8- against 4-wide pops, no window and window 72: 2048^2 15.9 and 14.0,
+// 14.6 and 13.4 ms; 2896^2 22.5 and 20.8, 20.6 and 20.2; 3200^2 25.4 and 23.8,
+// 22.9 and 23.3; 3500^2 28.3 and 27.2, 25.2 and 26.7; 4096^2, searches alone,
+// 34.3 and 34.8, 31.0 and 34.0.  Hence the line at 2^23 cells (2896^2).
 // Q above 16384 asks for throughput on hard puzzles: pops as wide as it says.
 inline PlainShape ring_shape(uint32_t sms, uint32_t kind, uint64_t cells, const gastar_config& cfg, uint64_t Q) {
     PlainShape s;
     const uint64_t warps = 8ull * sms;
     s.W = cfg.warps_per_block ? std::min(16u, cfg.warps_per_block) : 8u;
     if (cfg.expansion_width) s.ew = std::min(32u, cfg.expansion_width);
-    else if (kind == KIND_GRID) s.ew = cells >= (1ull << 22) ? 8 : 4;
+    else if (kind == KIND_GRID) s.ew = cells >= (1ull << 23) ? 8 : 4;
     else s.ew = (uint32_t)std::min<uint64_t>(Q <= 16384 ? 8 : 32, std::max<uint64_t>(4, (Q + warps - 1) / warps));
     const bool fixed = cfg.expansion_width || cfg.warps_per_block;
     const uint64_t heaps = std::min<uint64_t>((Q + s.ew - 1) / s.ew, fixed ? ~0ull : warps);
@@ -68,9 +71,10 @@ inline PlainShape ring_shape(uint32_t sms, uint32_t kind, uint64_t cells, const 
 // fences and flags (~2400), but have a tenth of the SMs: taken for searches
 // whose iterations hold a few hundred entries -- Q that small, 8-puzzles
 // (181,440 states in all; 0.167 against 0.196 ms) and grids up to 2^17 cells
-// (200 x 150: 0.92 against 1.12 ms; 360 x 360: 2.18 against 2.13; 517 x 389:
-// 3.03 against 2.81).  resident(warps, ew, blocks): whether a cluster of that
-// many blocks of that shape fits on the GPU.
+// (means of two grids, cluster and ring: 200^2 1.06 and 1.24 ms, 300^2 1.70
+// and 1.88, 362^2 2.21 and 2.31; 420^2 2.79 and 2.67, 512^2 3.82 and 3.32).
+// resident(warps, ew, blocks): whether a cluster of that many blocks of that
+// shape fits on the GPU.
 template <class Resident>
 PlainShape cluster_shape(uint32_t kind, uint64_t cells, const gastar_config& cfg, uint64_t Q, Resident resident) {
     PlainShape s;
