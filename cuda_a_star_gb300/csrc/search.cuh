@@ -264,7 +264,6 @@ struct GridDom {
     static __device__ __forceinline__ uint32_t start_f(const Ctx&, const InstDesc& d) { return d.f0; }
     static constexpr uint32_t kRootCode = kRootMove;
     static constexpr bool kParentBySlot = false;
-    static __device__ __forceinline__ uint32_t code(int m, uint32_t) { return (uint32_t)m; }
     static constexpr bool kDense = true;
     // The cell is the slot: one atomicMin claims and lowers it.
     static __device__ __forceinline__ uint64_t lower(const Tab& t, KeyT k, uint64_t v) {
@@ -1021,8 +1020,8 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
                 // precedes everything after (acquire).
                 fence_acq_rel_gpu();
                 red_relaxed_add_u32(&c->count, 1u);
-                sm.agg.err = sm.agg.claims = sm.agg.exps = sm.agg.perr = 0;  // not the count
-                sm.agg.minstage = sm.agg.best = sm.agg.minheap = kInf;
+                sm.agg.err = sm.agg.claims = sm.agg.exps = 0;  // not the count
+                sm.agg.minstage = sm.agg.best = kInf;
                 sm.agg_minheap = kInf;
                 sm.agg_err_prev = 0;
                 uint32_t dec = kInf, dbest = kInf, dfmin = kInf;
