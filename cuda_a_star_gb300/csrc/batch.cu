@@ -140,7 +140,7 @@ struct gastar_batch {
     uint32_t n_heavy = 0, heavy_teams = 0;
     uint64_t heavy_stage_bytes = 0;
     bool cluster = false;        // its teams are thread-block clusters
-    uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap nodes per warp
+    uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap places per warp + 1
     DevBuf team_ctl, team_stage;
     uint32_t promoted = 0;
     float main_ms = 0, retry_ms = 0, promote_ms = 0;  // kernel time by phase of the last run

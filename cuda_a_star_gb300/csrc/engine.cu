@@ -1,8 +1,9 @@
 // Host runtime and C ABI of the GA* engine (libgastar.so).
 //
-// Plain mode  : one instance per launch; a team of thread blocks (cooperative
-//               launch, device-side barriers) runs the whole search without a
-//               host round trip.  Replaces a_star() (a_star.h:223-282).
+// Plain mode  : one instance per launch; a team of thread blocks (one block,
+//               one cluster, or a ring of blocks in a cooperative launch) runs
+//               the whole search without a host round trip.  Replaces a_star()
+//               (a_star.h:223-282).
 // Batch mode  : many instances in one persistent launch, one block per
 //               instance at a time, per-instance table/heap partitions.
 #include <cuda_runtime.h>

@@ -20,8 +20,8 @@ constexpr uint32_t kind_bit(uint32_t k) { return 1u << k; }
 
 // Entries one stage buffer must hold: every popped entry of every warp-heap
 // can stage all of its successors.  Dynamic shared memory of one block holds
-// two stage buffers (one-block teams only) followed by the shared-memory heap
-// nodes of every warp.
+// two stage buffers (one-block and cluster teams) followed by the
+// shared-memory heap nodes of every warp.
 inline __host__ __device__ size_t stage_entries_per_buffer(uint32_t heaps, uint32_t ew, uint32_t maxn) {
     return (size_t)heaps * ew * maxn;
 }
@@ -58,13 +58,14 @@ constexpr uint32_t kWideAfter = 64;
 constexpr uint32_t kTouchedChunk = 1024;
 constexpr uint32_t kTouchedHole = 0xffffffffu;
 
-// Warp-heap nodes below sn live in shared memory (node 0 in registers).
-constexpr uint32_t kHeapSmemNodes = 7;      // default sn: nodes 1..6
+// 32-entry places per warp in shared memory, plus one: the heap's partial
+// buffer, then its nodes from the root on.
+constexpr uint32_t kHeapSmemNodes = 7;      // default: the buffer and nodes 0..4
 // Dynamic shared memory above this needs the opt-in attribute: a block's
 // static shared memory (the kernels' CtaShared, ~1.2 KB) counts against the
 // default 48 KiB as well.
 constexpr size_t kSmemNoOptIn = 44 * 1024;
-constexpr uint32_t kHeapSmemNodesMax = 127;  // levels 0..6
+constexpr uint32_t kHeapSmemNodesMax = 127;  // levels 0..5 and most of 6
 // Global stage area of a multi-block team: kStageRing buffers, each one
 // region of warps*ew*maxn entries per block; then one 64-bit ready word per
 // region (kStageRing rows of `blocks` words): (iteration + 1) << 32 | the
@@ -208,7 +209,7 @@ struct LaunchParams {
     const uint32_t* order;    // schedule order (nullptr = 0..n-1)
     uint32_t* next;           // work counter for single-block teams
     uint32_t team_ctas;       // 1 = one block per instance; >1 = all blocks on instance 0
-    uint32_t heap_snodes;     // shared-memory heap nodes per warp + 1 (0 = kHeapSmemNodes)
+    uint32_t heap_snodes;     // shared-memory heap places per warp + 1 (0 = kHeapSmemNodes)
     uint32_t buckets;         // 1 = blocks carry the bucket push scratch (some instance has buckets)
     uint32_t cluster;         // 1 = the blocks of a team are one thread-block cluster
     TeamCtl* team;            // multi-block team control (device)

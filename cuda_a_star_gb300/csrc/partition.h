@@ -41,7 +41,7 @@ struct PartConfig {
     uint64_t max_exp = 0;
     uint32_t timeout_ms = 0;
     uint32_t retry_level = 0;     // capacities scale by 4^retry_level
-    uint32_t heap_snodes = kHeapSmemNodes;  // heap nodes below this index live in shared memory
+    uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap places per warp + 1
     bool buckets = false;         // bucket front in front of the warp-heaps
     bool own_weights = false;     // grid weights live inside the partition
     bool claim_list = false;      // puzzles: record claimed slots so that the next search

@@ -762,13 +762,14 @@ __device__ __noinline__ void run_instance(const LaunchParams& P, const TeamRef t
         // Lane l of round r takes move l % LPE of entry r * EPR + l / LPE.
         // Bound by round trips to L2/HBM and by the SM's rate of scattered
         // accesses (measured per SM: one L2 load per cycle, one L2 atomic per
-        // 2.1, six cycles per random HBM sector); per round one probe
+        // 2.1, seven cycles per random HBM sector); per round one probe
         // instruction covers EPR whole neighbourhoods (a grid cell's three
         // rows share sectors), RB rounds' probes are in flight together, and
         // a warp that popped few entries runs few rounds.  A plain 4096^2
         // grid pops four entries per warp and iteration: with one lane per
         // entry and the moves in sequence its expansion took 8.9 k cycles of
-        // a 27 k cycle iteration, now 3.1 k of 18 k (74.4 -> 48.9 ms).  The
+        // a 27 k cycle iteration; this alone took it from 74.4 to 48.9 ms, and
+        // it is 3.4 k of 11.4 k cycles now (31 ms).  The
         // lane of the move straight back to the parent, which has no
         // successor, checks whether the entry is stale.
         const uint32_t live = __ballot_sync(kFull, act);
@@ -1328,8 +1329,9 @@ __device__ __forceinline__ void dispatch(const LaunchParams& P, const TeamRef tm
 
 // The block's next instance into its shared state; false: none is left.  A
 // function of its own so that nothing of it, hoisted out of the caller's loop,
-// holds registers across a search: the 16-warp kernel's searches spilled 120
-// bytes for grids and 132 for boards with it in the loop, 8 and 44 without.
+// holds registers across a search: the 16-warp kernel's one-block searches
+// spilled 120 bytes for grids and 132 for boards with it in the loop, 8 and 44
+// without (spill loads; 24-puzzles 228, ring-team grids 68).
 inline __device__ __noinline__ bool take_instance(const LaunchParams& P) {
     CtaShared& sm = cta();
     if (threadIdx.x == 0) sm.inst = atomicAdd(P.next, 1u);

@@ -105,7 +105,7 @@ struct gastar_server {
     uint32_t resident = 0;      // blocks resident on the device at once
     uint32_t clusters = 0;      // clusters of heavy_team blocks resident at once (0: no such clusters)
     uint64_t heavy_stage_bytes = 0;
-    uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap nodes per warp
+    uint32_t heap_snodes = kHeapSmemNodes;  // shared-memory heap places per warp + 1
     RangeAlloc alloc;  // the arena
     uint32_t max_active = 0, threads = 0;
     size_t smem = 0;

@@ -73,7 +73,9 @@ typedef struct gastar_config {
     uint64_t max_expansions;   /* 0 = unlimited */
     uint32_t max_iterations;   /* 0 = unlimited */
     uint32_t timeout_ms;       /* device-side deadline, 0 = none */
-    uint32_t regrow;           /* plain engine: re-run with doubled capacity on *_FULL (default 1) */
+    uint32_t regrow;           /* plain engine: re-run with larger capacity on *_FULL (default 1):
+                                  eight times the table's slots, or as many as fit; twice
+                                  the heaps' entries */
     uint32_t delta;            /* pop window: expand only f <= min f + delta (0 = no window) */
     uint32_t open_list;        /* 0 = warp-heaps (top levels in shared memory);
                                   1 = shared-memory f-buckets in front of the warp-heaps */
