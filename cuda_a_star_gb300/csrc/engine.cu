@@ -497,7 +497,7 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
                                     return occupancy_clusters(kinds, warps * 32, smem, blocks) >= 1;
                                 });
     const uint32_t ew = sh.ew, W = sh.W, threads = W * 32;
-    size_t smem = block_smem_bytes(kinds, W, ew, sh.ring());
+    size_t smem = block_smem_bytes(kinds, W, sh.ew_wide, sh.ring());
     const int nb = occupancy_blocks(c, kinds, threads, smem);
     if (nb <= 0) return GASTAR_CUDA_ERROR;
     sh.blocks = std::min(sh.blocks, (uint64_t)nb * c->sms);
@@ -507,10 +507,10 @@ static int plain_attempt(gastar_ctx* c, const PlainProblem& pp, const gastar_con
     const uint32_t ew_wide = sh.ew_wide;
     // The shared memory the co-resident blocks leave free holds the heaps' top
     // levels: pops and pushes then touch global nodes only deep down.
-    uint32_t snodes = fit_heap_snodes(c, kinds, W, ew, ring, threads,
-                                            (int)((blocks + c->sms - 1) / c->sms), &smem, buckets);
+    uint32_t snodes = fit_heap_snodes(c, kinds, W, ew_wide, ring, threads,
+                                      (int)((blocks + c->sms - 1) / c->sms), &smem, buckets);
     if (cluster && occupancy_clusters(kinds, threads, smem, (uint32_t)blocks) < 1) {
-        smem = block_smem_bytes(kinds, W, ew, ring, kHeapSmemNodes, buckets);
+        smem = block_smem_bytes(kinds, W, ew_wide, ring, kHeapSmemNodes, buckets);
         snodes = kHeapSmemNodes;
     }
     if (ring && !c->coop) {

@@ -39,6 +39,18 @@ struct PlainShape {
     bool ring() const { return blocks > 1 && !cluster; }
 };
 
+// Pops per warp-heap of a widened search.  A puzzle search with the automatic
+// width that passes kWideAfter iterations is a hard one, whose iteration count
+// the pops per iteration set rather than its depth; from then on every
+// warp-heap pops four times as many (at most 32).  On the 64 15-puzzles of the
+// plain benchmark (Q = 16384, 8-wide pops) the hardest took 333 iterations with
+// twice the pops and takes 206 with four times; the 64 together 4 % less time.
+// 12 15-puzzles on clusters (Q = 512, 256, 128) 24.0, 44.6 and 86.3 ms without
+// it, 14.8, 23.3 and 42.3 with it; the hardest 9.4 and 4.6 at Q = 512.
+inline uint32_t widened(const PlainShape& s, uint32_t kind, const gastar_config& cfg) {
+    return s.blocks > 1 && kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 4 * s.ew) : s.ew;
+}
+
 // Shape of a ring team with the automatic widths: eight warps on every SM,
 // popping few entries each.  An iteration lasts as long as its slowest warp,
 // and a warp expands its pops in rounds (four grid cells, eight boards), so
@@ -73,7 +85,7 @@ inline PlainShape ring_shape(uint32_t sms, uint32_t kind, uint64_t cells, const 
 // (181,440 states in all; 0.167 against 0.196 ms) and grids up to 2^17 cells
 // (means of two grids, cluster and ring: 200^2 1.06 and 1.24 ms, 300^2 1.70
 // and 1.88, 362^2 2.21 and 2.31; 420^2 2.79 and 2.67, 512^2 3.82 and 3.32).
-// resident(warps, ew, blocks): whether a cluster of that many blocks of that
+// resident(warps, widest pop, blocks): whether a cluster of that many blocks of that
 // shape fits on the GPU.
 template <class Resident>
 PlainShape cluster_shape(uint32_t kind, uint64_t cells, const gastar_config& cfg, uint64_t Q, Resident resident) {
@@ -90,19 +102,9 @@ PlainShape cluster_shape(uint32_t kind, uint64_t cells, const gastar_config& cfg
     }
     if (cfg.max_blocks) blocks = std::min<uint64_t>(blocks, cfg.max_blocks);
     s.cluster = blocks > 1;
-    if (s.cluster && !resident(s.W, s.ew, (uint32_t)blocks)) return PlainShape();
     s.blocks = blocks;
+    if (s.cluster && !resident(s.W, widened(s, kind, cfg), (uint32_t)blocks)) return PlainShape();
     return s;
-}
-
-// Pops per warp-heap of a widened search.  A puzzle search with the automatic
-// width that passes kWideAfter iterations is a hard one, whose iteration count
-// the pops per iteration set rather than its depth; from then on every
-// warp-heap pops four times as many (at most 32).  On the 64 15-puzzles of the
-// plain benchmark (Q = 16384, 8-wide pops) the hardest took 333 iterations with
-// twice the pops and takes 206 with four times; the 64 together 4 % less time.
-inline uint32_t widened(const PlainShape& s, uint32_t kind, const gastar_config& cfg) {
-    return s.ring() && kind != KIND_GRID && !cfg.expansion_width ? std::min(32u, 4 * s.ew) : s.ew;
 }
 
 // The team of a solve: a cluster where one is taken, else a ring; one block

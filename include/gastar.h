@@ -61,7 +61,7 @@ typedef struct gastar_config {
     uint32_t expansion_width;  /* entries each warp-heap pops per iteration, 1..32;
                                   0 = auto, 4 to 8 on up to eight warps per SM
                                   (puzzles above 16384 queues: up to 32), and a
-                                  puzzle search on many blocks that passes 64
+                                  puzzle search on several blocks that passes 64
                                   iterations then pops four times as many (at most 32) */
     uint32_t warps_per_block;  /* warp-heaps per thread block, 1..16 (above 8: the
                                   512-thread kernel, at most 128 registers per thread);

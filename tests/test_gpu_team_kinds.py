@@ -84,3 +84,17 @@ def test_requests_go_from_clusters_to_rings_and_back(engine, oracle, gastar):
     for i in heavy:
         h, w = grids[i].shape
         assert oracle.grid_validate(grids[i], (0, 0), (w - 1, h - 1), got[i].path) == (True, want[i])
+
+
+@pytest.mark.parametrize("queues", [64, 512])
+def test_clusters_widen(engine, oracle, gastar, queues):
+    """A puzzle that is past 64 iterations on a cluster takes fewer of them with
+    the automatic width than with that width fixed."""
+    s, g = gastar.gen_sliding(4, 909, 40, 70)
+    want = oracle.sliding_astar(4, s, g, path=False)[0].cost
+    auto = engine.solve_sliding(s, g, 4, num_queues=queues)
+    fixed = engine.solve_sliding(s, g, 4, num_queues=queues, expansion_width=4, warps_per_block=8)
+    for r in (auto, fixed):
+        assert r.status_name == "OK" and r.cost == want
+        assert oracle.sliding_validate(4, s, g, r.path) == (True, want)
+    assert fixed.iterations > 128 and auto.iterations < fixed.iterations

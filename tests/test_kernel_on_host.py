@@ -80,10 +80,11 @@ def test_costs_under_random_interleavings(search, gastar, oracle, team, blocks, 
         assert (r["launches"] > 1) == (slice > 0)
 
 
-def test_widened_rings(search, gastar, oracle):
+@pytest.mark.parametrize("team", [CLUSTER, RING])
+def test_widened_searches(search, gastar, oracle, team):
     for seed in range(4):
         inst, cost = _board(gastar, oracle, 4, 20 + seed, 26)
-        r = _run(search, inst, RING, 3, 2, 2, seed=seed, wide=(8, 4))
+        r = _run(search, inst, team, 3, 2, 2, seed=seed, wide=(8, 4))
         assert r.get("status") == STATUS["OK"] and r["cost"] == cost, r
 
 

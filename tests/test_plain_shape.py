@@ -34,10 +34,10 @@ int main() {
                                 const PlainShape s = plain_shape(sms, kind, cells, c,
                                                                  [&](uint32_t, uint32_t, uint32_t) { return resident != 0; });
                                 const uint32_t snodes = 20;
-                                std::printf("%u %u %u %u %u %u %llu %d %d %zu %zu\n", kind, cap, w, s.ew, s.ew_wide, s.W,
+                                std::printf("%u %u %u %u %u %u %u %llu %d %d %zu %zu\n", kind, cap, w, ew, s.ew, s.ew_wide, s.W,
                                             (unsigned long long)s.blocks, (int)s.cluster, (int)s.ring(),
-                                            block_smem_bytes(kind_bit(kind), s.W, s.ew, s.ring(), snodes, false),
-                                            block_smem_bytes(kind_bit(kind), s.W, s.ew, s.ring(), snodes, true));
+                                            block_smem_bytes(kind_bit(kind), s.W, s.ew_wide, s.ring(), snodes, false),
+                                            block_smem_bytes(kind_bit(kind), s.W, s.ew_wide, s.ring(), snodes, true));
                             }
         }
 }
@@ -56,17 +56,18 @@ def shapes(tmp_path_factory):
 
 
 def test_blocks_lie_within_the_cap_and_the_kind_follows_them(shapes):
-    assert any(s[8] for s in shapes) and any(s[7] for s in shapes)
-    for kind, cap, w, ew, ew_wide, W, blocks, cluster, ring, _, _ in shapes:
+    assert any(s[9] for s in shapes) and any(s[8] for s in shapes)
+    for kind, cap, w, fixed, ew, ew_wide, W, blocks, cluster, ring, _, _ in shapes:
         assert blocks >= 1 and 1 <= W <= 16 and 1 <= ew <= ew_wide <= 32
         assert not cap or blocks <= cap
         assert ring == (blocks > 1 and not cluster)
         assert not cluster or 2 <= blocks <= 16 and W <= 8
-        assert ew_wide == ew or ring
+        # Puzzles with the automatic width widen on several blocks, clusters too.
+        assert ew_wide == (min(32, 4 * ew) if blocks > 1 and kind < 3 and not fixed else ew)
 
 
 def test_shared_memory_holds_what_the_kernel_lays_out(shapes):
-    for kind, cap, w, ew, ew_wide, W, blocks, cluster, ring, heaps, buckets in shapes:
+    for kind, cap, w, fixed, ew, ew_wide, W, blocks, cluster, ring, heaps, buckets in shapes:
         entry, maxn = (32 if kind == 2 else 16), (8 if kind == 3 else 4)
         in_smem = blocks == 1 or cluster  # by the launch: team_ctas, cluster
         stage = 2 * W * max(ew, ew_wide) * maxn * entry if in_smem else 0
