@@ -402,7 +402,7 @@ int batch_upload(gastar_batch* b) {
     // An upload that failed further on left its arena: taken again as it is.
     if (b->arena.n < arena_bytes) c->batch_memory.give(b->arena, c->stream);
     if (!b->arena.p) {
-        if (!c->batch_memory.room(arena_bytes + (64ull << 20))) {
+        if (!c->batch_memory.room(arena_bytes, 64ull << 20)) {
             set_error("batch partitions exceed free device memory");
             return GASTAR_OUT_OF_MEMORY;
         }

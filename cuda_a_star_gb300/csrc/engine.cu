@@ -83,16 +83,12 @@ bool BatchMemory::take(DevBuf& b, size_t bytes, cudaStream_t st) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
-        uint64_t keep = kKeepMax;
         if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return false;
         props.location.id = dev;
         if (!cuda_ok(cudaMemPoolCreate(&pool_, &props), "cudaMemPoolCreate")) {
             pool_ = nullptr;
             return false;
         }
-        if (!cuda_ok(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep),
-                     "cudaMemPoolSetAttribute"))
-            return false;
     }
     void* p = nullptr;
     if (cudaMallocFromPoolAsync(&p, bytes, pool_, st) != cudaSuccess) {
@@ -105,6 +101,7 @@ bool BatchMemory::take(DevBuf& b, size_t bytes, cudaStream_t st) {
     b.p = p;
     b.n = bytes;
     b.fresh = b.pooled = true;
+    live_ += bytes;
     return true;
 }
 
@@ -116,6 +113,10 @@ void BatchMemory::give(DevBuf& b, cudaStream_t st) {
         b.release();
         return;
     }
+    // What batches still hold counts against the pool's threshold too.
+    live_ -= b.n;
+    uint64_t keep = live_ + kKeepMax;
+    cuda_ok(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
     cuda_ok(cudaFreeAsync(b.p, st), "cudaFreeAsync");
     cuda_ok(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     b = DevBuf();
@@ -132,15 +133,17 @@ void BatchMemory::close() {
     pool_ = nullptr;
 }
 
-bool BatchMemory::room(size_t bytes) {
+bool BatchMemory::room(size_t bytes, size_t beside) {
     std::lock_guard<std::mutex> lk(mu_);
     size_t free_b = 0, total_b = 0;
     uint64_t held = 0, used = 0;
-    cudaMemGetInfo(&free_b, &total_b);
     if (pool_) {
         cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &held);
         cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrUsedMemCurrent, &used);
     }
+    if (bytes <= held - used) return true;  // nothing of the device's (cudaMemGetInfo takes 18 us)
+    bytes += beside;
+    cudaMemGetInfo(&free_b, &total_b);
     if (bytes <= free_b + (held - used)) return true;
     void* p = nullptr;  // other contexts' pools: what cudaMalloc gets of them
     if (cudaMalloc(&p, bytes) != cudaSuccess) {

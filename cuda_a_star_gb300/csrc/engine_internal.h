@@ -26,8 +26,8 @@ struct DevBuf {
 // Device memory for batches that a context's later batches use again: mapping
 // and unmapping a batch's partitions (11 GB for 512 8-puzzles: 1.3 and 4.9 ms)
 // takes longer than searching them (1.9 ms).  What a destroyed batch gives back
-// stays in a memory pool of the driver, at most kKeepMax bytes, which hands it
-// out in exact sizes and takes it back by itself for any cudaMalloc of the
+// stays in a memory pool of the driver, at most kKeepMax bytes unused, which hands
+// it out in exact sizes and takes it back by itself for any cudaMalloc of the
 // process that would fail, whoever calls it (20 ms for 8 GB).  Growing a pool
 // takes longer than cudaMalloc (0.8 against 0.1 ms per GB, and 0.4 to free), so
 // the first batch of a context, and buffers above kKeepMax, go without it.
@@ -38,10 +38,10 @@ public:
     bool take(DevBuf& b, size_t bytes, cudaStream_t st);
     // Releases `b`; the work that used it is done.
     void give(DevBuf& b, cudaStream_t st);
-    // Whether a batch may take `bytes`: what is kept unused, here or by other
-    // contexts of the process, counts as free; the latter's is free after it
-    // where it was needed.
-    bool room(size_t bytes);
+    // Whether a batch may take `bytes`, and `beside` more of the device where it
+    // is not kept here: what other contexts of the process keep unused counts as
+    // free, and is free afterwards where it was needed.
+    bool room(size_t bytes, size_t beside);
     // Gives what is kept unused back to the device.
     void trim();
     void close();
@@ -50,6 +50,7 @@ private:
     std::mutex mu_;
     cudaMemPool_t pool_ = nullptr;
     bool again_ = false;  // a batch has been destroyed
+    uint64_t live_ = 0;   // bytes of the pool that batches hold
 };
 
 void set_error(const std::string& s);

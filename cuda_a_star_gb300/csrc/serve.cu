@@ -333,7 +333,7 @@ gastar_server* gastar_serve_create(gastar_ctx* c, const gastar_serve_config* cfg
     // The budget is a share of the memory that is free, what contexts keep
     // for batches included.
     c->batch_memory.trim();
-    c->batch_memory.room(budget + (2ull << 30));
+    c->batch_memory.room(budget, 2ull << 30);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     budget = std::min<uint64_t>(budget, free_b > (2ull << 30) ? free_b - (2ull << 30) : free_b / 2);

@@ -196,3 +196,21 @@ def test_a_regrown_table_far_larger_than_needed_is_not_kept(gastar, oracle):
         r = eng.solve_sliding(s, g, 4, heuristic=gastar.H_ZERO, **kw)
         assert r.cost == want and r.attempts == 2
         assert abs(_free() - before) < 256 * MIB
+
+
+def test_a_resident_batch_does_not_shrink_what_is_kept(gastar):
+    """8.6 GB in a resident batch and 11.5 GB kept for the next: over the 16 GiB
+    that are kept unused only together."""
+    with gastar.Engine(0) as eng:
+        for _ in range(2):
+            b = _puzzles(eng, gastar, 80)
+            b.run()
+            b.close()
+        resident = _puzzles(eng, gastar, 60)
+        resident.run()
+        b = _puzzles(eng, gastar, 80)
+        b.run()
+        held = _free()
+        b.close()
+        assert _free() < held + 512 * MIB
+        resident.close()
